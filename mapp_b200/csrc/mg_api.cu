@@ -450,7 +450,7 @@ int ensure_atoms(mg_system* s, size_t need, size_t keep)
     return MG_OK;
 }
 
-// ELL list storage; EAM / FS keep their two per-pair derivatives in ELL slots
+// ELL list storage
 int ensure_pairs(mg_system* s, int maxnb)
 {
     Dev& d = s->d;
@@ -458,15 +458,13 @@ int ensure_pairs(mg_system* s, int maxnb)
     if (np > s->nbr_cap) {
         size_t cap = np + np / 4 + 1024;
         CHK(dalloc(&d.nbr, cap));
-        if (!s->dmd) CHK(dalloc(&d.pr, cap * s->npair_blocks));
         s->nbr_cap = cap;
     }
     d.maxnb = maxnb;
-    if (!s->dmd) d.maxp = (long long)np;
     return MG_OK;
 }
 
-// compact pair list and (DMD) per-pair scratch for npairs pairs
+// compact pair list and the per-pair scratch for npairs pairs
 int ensure_compact(mg_system* s, long long npairs)
 {
     Dev& d = s->d;
@@ -474,10 +472,10 @@ int ensure_compact(mg_system* s, long long npairs)
     long long cap = npairs + npairs / 5 + 1024;
     CHK(dalloc(&d.pair_i, (size_t)cap));
     CHK(dalloc(&d.pair_j, (size_t)cap));
+    CHK(dalloc(&d.pr, (size_t)cap * s->npair_blocks));
+    d.maxp = cap;
     if (s->dmd) {
-        CHK(dalloc(&d.pr, (size_t)cap * s->npair_blocks));
         CHK(dalloc(&d.prf, (size_t)cap * s->npair_blocks));
-        d.maxp = cap;
         d.icut_cap = dmd32_icut_capacity(cap);
         CHK(dalloc(&d.icut, (size_t)d.icut_cap * 2));
         if (!d.icut_n) CHK(dalloc(&d.icut_n, (size_t)dmd32_icut_warps()));
@@ -911,6 +909,28 @@ int upload_tables(mg_system* s)
     d.rhoT = s->d_rhoT;
     d.phiT = s->d_phiT;
     d.FT = s->d_FT;
+    {
+        // {rho c0..c3, phi c0..c3} per ordered species pair (a, b) and knot,
+        // coefficients copied unchanged: the density slot is b*nt+a for the DMD
+        // forms, with phi for a >= b, and the one EAM reads for an atom of type a
+        // with a neighbour of type b
+        const int nt = s->nt, nr = s->nr;
+        std::vector<double> pk64((size_t)nt * nt * nr * 8, 0.0);
+        for (int a = 0; a < nt; a++)
+            for (int b = 0; b < nt; b++)
+                for (int m = 0; m < nr; m++) {
+                    double* dst = pk64.data() + (((size_t)(a * nt + b) * nr + m) * 8);
+                    const double* rr = s->rhoT.data() + ((size_t)(s->dmd ? b * nt + a : a * nt + b) * nr + m) * 8;
+                    for (int k = 0; k < 4; k++) dst[k] = rr[k];
+                    if (a >= b || !s->dmd) {
+                        const double* pp = s->phiT.data() + ((size_t)comp_idx(a, b) * nr + m) * 8;
+                        for (int k = 0; k < 4; k++) dst[4 + k] = pp[k];
+                    }
+                }
+        CHK(dalloc(&s->d_pk64, pk64.size()));
+        CU(cudaMemcpy(s->d_pk64, pk64.data(), pk64.size() * sizeof(double), cudaMemcpyHostToDevice));
+        d.pk64 = s->d_pk64;
+    }
     if (s->dmd) {
         // precision form: {rho c0..c3 of slot b*nt+a, phi c0..c3 of COMP(a,b)} per (a,b) and knot
         int nt = s->nt, nr = s->nr;
@@ -929,22 +949,6 @@ int upload_tables(mg_system* s)
         CHK(dalloc(&s->d_pkT, pk.size()));
         CU(cudaMemcpy(s->d_pkT, pk.data(), pk.size() * sizeof(float), cudaMemcpyHostToDevice));
         d.pkT = reinterpret_cast<const float4*>(s->d_pkT);
-        // plain form: the same pairing, coefficients copied unchanged
-        std::vector<double> pk64((size_t)nt * nt * nr * 8, 0.0);
-        for (int a = 0; a < nt; a++)
-            for (int b = 0; b < nt; b++)
-                for (int m = 0; m < nr; m++) {
-                    double* dst = pk64.data() + (((size_t)(a * nt + b) * nr + m) * 8);
-                    const double* rr = s->rhoT.data() + ((size_t)(b * nt + a) * nr + m) * 8;
-                    for (int k = 0; k < 4; k++) dst[k] = rr[k];
-                    if (a >= b) {
-                        const double* pp = s->phiT.data() + ((size_t)comp_idx(a, b) * nr + m) * 8;
-                        for (int k = 0; k < 4; k++) dst[4 + k] = pp[k];
-                    }
-                }
-        CHK(dalloc(&s->d_pk64, pk64.size()));
-        CU(cudaMemcpy(s->d_pk64, pk64.data(), pk64.size() * sizeof(double), cudaMemcpyHostToDevice));
-        d.pk64 = s->d_pk64;
         // The precision form's shared-memory table: kSplitKnots knots over
         // [0, rc], each interval the cubic Hermite piece through the fine
         // spline's value and slope at its ends (fine interpolant evaluated as in
@@ -1690,8 +1694,7 @@ int mg_ff_fin(mg_system* s)
     if (d.pr) cudaFree(d.pr);
     d.pr = nullptr;
     d.maxp = 0;
-    if (s->dmd) s->pair_cap = 0;
-    else s->nbr_cap = 0;  // EAM / FS keep their pair derivatives beside the ELL list
+    s->pair_cap = 0;
     s->initialized = false;
     s->crd_built = 0;
     return MG_OK;

@@ -102,22 +102,6 @@ __device__ __forceinline__ float2 seg_sum2(float v, const Seg& s)
     return make_float2(hi, lo);
 }
 
-// Segments of a warp whose keys are sorted (equal keys in contiguous lanes,
-// padding lanes with key -1 at the end): boundaries from one shuffle and one
-// ballot instead of a match instruction.
-__device__ __forceinline__ Seg seg_sorted(int key)
-{
-    const int lane = threadIdx.x & 31;
-    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != key);
-    const unsigned upto = heads & (0xffffffffu >> (31 - lane));  // heads at or before this lane
-    const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
-    Seg sg;
-    sg.first = 31 - __clz(upto);
-    sg.last = after ? __ffs(after) - 2 : 31;
-    return sg;
-}
-
 // FP32 sum over the caller's segment (first lane of the segment receives it)
 __device__ __forceinline__ float seg_sumf(float v, const Seg& s)
 {

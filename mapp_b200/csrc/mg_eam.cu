@@ -1,136 +1,133 @@
 // Tabulated EAM (ff_eam.cpp:44-356) and analytic Finnis-Sinclair
 // (ff_fs.cpp:379-684) force / energy kernels.
 //
-// Layout of work: one warp per owned atom i, lanes stride over i's half list.
-// i-side sums (density, force) are warp-shuffle reductions finished with one
-// atomic per warp; j-side contributions are FP64 atomics on j (owned j only,
-// as in the reference: ghost j receive nothing and their pair energy and
-// virial count one half).  Energy and virial go to per-block partial rows
-// reduced deterministically at the end.
+// Layout of work: one lane per listed pair of the compact list (pairs sorted by
+// i), so every lane carries work however many neighbours an atom has.  The
+// forces and densities of a warp's pairs are added up through shared memory
+// (rows_scatter for the atoms j, rows_runs for the atoms i; owned j only, as in
+// the reference: ghost j receive nothing and their pair energy and virial count
+// one half).
+// Energy and virial go to per-block partial rows reduced deterministically at
+// the end; the grids are persistent, so there are a few thousand rows at most.
 //
-// Pass 1 stores -drho/dr / r for both sides of every pair (pair slot
-// i*maxnb+k) exactly like drhoi_dr / drhoj_dr (ff_eam.cpp:172-173); pass 2
-// reads F'(rho) of a ghost j from its owner (the ghost refresh
-// atoms->update(rho_n), ff_eam.cpp:194, fused into the load).
+// Pass 1 stores -drho/dr / r for both sides of every pair (one 16-byte item per
+// pair) like drhoi_dr / drhoj_dr (ff_eam.cpp:172-173); pass 2 reads F'(rho) of a
+// ghost j from its owner (the ghost refresh atoms->update(rho_n),
+// ff_eam.cpp:194, fused into the load).
+//
+// What bounds the pair passes: the L1 data stage takes one cycle per lane of a
+// gather (positions, 32-byte spline knots), per line of a reduction and per
+// shuffle.  With one warp per atom, two 64-byte knot rows, the species gather and
+// four single reductions a pair cost 10 of them and 256000 atoms took 380 us
+// (pass 1) and 286 us (pass 2); here the derivative comes from the value's
+// coefficients, one species needs no gather, and the reductions share lines:
+// 177 us and 115 us (L1 data stage 84 % and 76 % busy; 798 -> 352 us a call).
 #include "mg_reduce.cuh"
+#include "mg_dmd_common.cuh"
 
 namespace mg {
 
 namespace {
 
-__device__ __forceinline__ int owner(const Dev& d, int j) { return j < d.natms ? j : d.root[j]; }
-
-// One knot row of a spline table (8 doubles: c0..c3 of the value, c4..c6 of
-// the derivative, one pad) as two 32-byte read-only loads.
-struct Row8 {
-    double4 v, dv;
-};
-__device__ __forceinline__ Row8 row8(const double* __restrict__ row)
-{
-    Row8 r;
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.v.x), "=d"(r.v.y), "=d"(r.v.z), "=d"(r.v.w) : "l"(row));
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
-        : "=d"(r.dv.x), "=d"(r.dv.y), "=d"(r.dv.z), "=d"(r.dv.w)
-        : "l"(row + 4));
-    return r;
-}
-
-// Resident blocks per SM the EAM pass 1 is compiled for (64 registers a
-// thread at 4): a small system's warps then fit one wave.
+// Resident blocks per SM of the pair passes (64 registers a thread at 4).
 #ifndef MG_EAM_MINB
 #define MG_EAM_MINB 4
 #endif
 
-// EAM pass 1 (ff_eam.cpp:95-177).  energy_only skips forces and stored
-// derivatives (ForceField_eam::energy_calc, ff_eam.cpp:297-338).
-template <bool kEnergyOnly>
+// f(p, valid, i) for the compact pairs, a warp's lanes together
+template <typename F>
+__device__ __forceinline__ void for_pairs(const Dev& d, F f)
+{
+    const int lane = threadIdx.x & 31;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; b < d.npairs; b += stride) {
+        const long long p = b + lane;
+        const bool valid = p < d.npairs;
+        f(p, valid, valid ? d.pair_i[p] : -1);
+    }
+}
+
+// the sums of a warp's pairs: value q < 3 of a row is a force component, q = 3 a density
+__device__ __forceinline__ void add_value(const Dev& d, int row, int q, double x)
+{
+    atomicAdd(q < 3 ? d.f + (size_t)row * 3 + q : d.rho + row, x);
+}
+
+__device__ __forceinline__ void add_virial(double (&acc)[7], double w, double dx0, double dx1, double dx2)
+{
+    acc[1] -= w * dx0 * dx0;
+    acc[2] -= w * dx1 * dx1;
+    acc[3] -= w * dx2 * dx2;
+    acc[4] -= w * dx1 * dx2;
+    acc[5] -= w * dx2 * dx0;
+    acc[6] -= w * dx0 * dx1;
+}
+
+// EAM pass 1 (ff_eam.cpp:95-177).  kEnergyOnly skips forces and stored
+// derivatives (ForceField_eam::energy_calc, ff_eam.cpp:297-338); kOne: one
+// species, whose index is not read and whose two densities are the same.
+template <bool kEnergyOnly, bool kOne>
 __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_eam_pass1(Dev d, int st_clc, int row0)
 {
-    int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    constexpr int NV = kEnergyOnly ? 1 : 4;
+    __shared__ RowBuf<NV> sh[kFFWarps];
+    RowBuf<NV>& buf = sh[threadIdx.x >> 5];
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (i < d.natms) {
-        double4 xi = d.pos[i];
-        int ti = d.type[i];
-        int nt = d.nt;
-        double rho_i = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-        int nn = d.nnb[i];
-        for (int k = lane; k < nn; k += 32) {
-            long long slot = (long long)i * d.maxnb + k;
-            int j = d.nbr[slot];
-            int tj = d.type[j];
-            double4 xj = d.pos[j];
-            double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
-            double rsq = __dadd_rn(__dadd_rn(__dmul_rn(dx0, dx0), __dmul_rn(dx1, dx1)), __dmul_rn(dx2, dx2));
-            double pi_ = 0.0, pj_ = 0.0;
+    for_pairs(d, [&](long long p, bool valid, int i) {
+        // the pair's shares: of atom j its force and density (the other way round, of atom i)
+        double v[NV], rho_i = 0.0, pi_ = 0.0, pj_ = 0.0;
+#pragma unroll
+        for (int q = 0; q < NV; q++) v[q] = 0.0;
+        int row = -1;
+        if (valid) {
+            const int j = d.pair_j[p];
+            const double4 xi = d.pos[i], xj = d.pos[j];
+            const double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
+            const double rsq = __dadd_rn(__dadd_rn(__dmul_rn(dx0, dx0), __dmul_rn(dx1, dx1)), __dmul_rn(dx2, dx2));
             if (rsq < d.cut_sq) {
-                double r = sqrt(rsq);
-                double r_inv = 1.0 / r;
-                double p = r * d.dr_inv;
-                int m = min((int)p, d.nr - 2);
-                p -= m;
-                p = fmin(p, 1.0);
-                const Row8 cf = row8(d.rhoT + ((size_t)(ti * nt + tj) * d.nr + m) * 8);
-                double rho_iv = ((cf.v.w * p + cf.v.z) * p + cf.v.y) * p + cf.v.x;
-                double drho_i = (cf.dv.z * p + cf.dv.y) * p + cf.dv.x;
-                // the j-side density row is the same row when the species agree
-                const Row8 cg = tj == ti ? cf : row8(d.rhoT + ((size_t)(tj * nt + ti) * d.nr + m) * 8);
-                double rho_jv = ((cg.v.w * p + cg.v.z) * p + cg.v.y) * p + cg.v.x;
-                double drho_j = (cg.dv.z * p + cg.dv.y) * p + cg.dv.x;
-                const Row8 ch = row8(d.phiT + ((size_t)comp_idx(ti, tj) * d.nr + m) * 8);
-                double z2 = ((ch.v.w * p + ch.v.z) * p + ch.v.y) * p + ch.v.x;
-                double phi = z2 * r_inv;
-                rho_i += rho_iv;
-                bool own_j = j < d.natms;
-                if (own_j) atomicAdd(&d.rho[j], rho_jv);
-                double w = own_j ? 1.0 : 0.5;
+                const int ti = kOne ? 0 : d.type[i], tj = kOne ? 0 : d.type[j];
+                const double r = sqrt(rsq);
+                const double r_inv = 1.0 / r;
+                double q = r * d.dr_inv;
+                const int m = min((int)q, d.nr - 2);
+                q -= m;
+                q = fmin(q, 1.0);
+                // knots of rho(ti, tj) and phi side by side (Dev::pk64)
+                const double* kt = d.pk64 + ((size_t)(ti * d.nt + tj) * d.nr + m) * 8;
+                const double4 cf = knot4(kt), ch = knot4(kt + 4);
+                const double4 cg = kOne || tj == ti ? cf : knot4(d.pk64 + ((size_t)(tj * d.nt + ti) * d.nr + m) * 8);
+                const double rho_jv = ((cg.w * q + cg.z) * q + cg.y) * q + cg.x;
+                const double z2 = ((ch.w * q + ch.z) * q + ch.y) * q + ch.x;
+                const double phi = z2 * r_inv;
+                const bool own_j = j < d.natms;
+                const double w = own_j ? 1.0 : 0.5;
+                rho_i = kOne ? rho_jv : ((cf.w * q + cf.z) * q + cf.y) * q + cf.x;
+                v[NV - 1] = rho_jv;
+                if (own_j) row = j;
                 acc[0] += w * phi;
                 if (!kEnergyOnly) {
-                    double z2p = (ch.dv.z * p + ch.dv.y) * p + ch.dv.x;
-                    double dphi = z2p * r_inv - phi * r_inv;
-                    double fpair = -dphi * r_inv;
-                    fx += fpair * dx0;
-                    fy += fpair * dx1;
-                    fz += fpair * dx2;
-                    if (own_j) {
-                        double* fj = d.f + (size_t)j * 3;
-                        atomicAdd(fj + 0, -fpair * dx0);
-                        atomicAdd(fj + 1, -fpair * dx1);
-                        atomicAdd(fj + 2, -fpair * dx2);
-                    }
-                    if (st_clc) {
-                        double wf = w * fpair;
-                        acc[1] -= wf * dx0 * dx0;
-                        acc[2] -= wf * dx1 * dx1;
-                        acc[3] -= wf * dx2 * dx2;
-                        acc[4] -= wf * dx1 * dx2;
-                        acc[5] -= wf * dx2 * dx0;
-                        acc[6] -= wf * dx0 * dx1;
-                    }
-                    pi_ = -drho_i * r_inv;
-                    pj_ = -drho_j * r_inv;
+                    const double z2p = ((3.0 * ch.w * q + 2.0 * ch.z) * q + ch.y) * d.dr_inv;
+                    const double dphi = z2p * r_inv - phi * r_inv;
+                    const double fpair = -dphi * r_inv;
+                    v[0] = -fpair * dx0;
+                    v[1 % NV] = -fpair * dx1;
+                    v[2 % NV] = -fpair * dx2;
+                    if (st_clc) add_virial(acc, w * fpair, dx0, dx1, dx2);
+                    pj_ = -((3.0 * cg.w * q + 2.0 * cg.z) * q + cg.y) * d.dr_inv * r_inv;
+                    pi_ = kOne ? pj_ : -((3.0 * cf.w * q + 2.0 * cf.z) * q + cf.y) * d.dr_inv * r_inv;
                 }
             }
-            if (!kEnergyOnly) {
-                d.pr[slot] = pi_;
-                d.pr[d.maxp + slot] = pj_;
-            }
+            if (!kEnergyOnly) __stcs(reinterpret_cast<double2*>(d.pr) + p, make_double2(pi_, pj_));
         }
-        rho_i = warp_sum(rho_i);
-        if (!kEnergyOnly) {
-            fx = warp_sum(fx);
-            fy = warp_sum(fy);
-            fz = warp_sum(fz);
+        rows_put<NV>(buf, v, i);
+        rows_scatter<NV>(buf, row, [&](int r, int q, double x) { add_value(d, r, q + 4 - NV, x); });
+        if (!kOne) {  // atom i's density is not atom j's
+            __syncwarp();
+            buf.v[(threadIdx.x & 31) * RowBuf<NV>::PITCH + NV - 1] = rho_i;
+            __syncwarp();
         }
-        if (lane == 0) {
-            atomicAdd(&d.rho[i], rho_i);
-            if (!kEnergyOnly) {
-                atomicAdd(d.f + (size_t)i * 3 + 0, fx);
-                atomicAdd(d.f + (size_t)i * 3 + 1, fy);
-                atomicAdd(d.f + (size_t)i * 3 + 2, fz);
-            }
-        }
-    }
+        rows_runs<NV>(buf, [&](int r, int q, double x) { add_value(d, r, q + 4 - NV, q + 4 - NV < 3 ? -x : x); });
+    });
     block_partials<7>(acc, d.partial, row0 + blockIdx.x);
 }
 
@@ -159,140 +156,97 @@ __global__ void __launch_bounds__(kFFBlock) k_eam_embed(Dev d, int row0)
 
 // EAM / FS pass 2: embedding forces from the stored pair derivatives
 // (ff_eam.cpp:196-250, ff_fs.cpp:531-588).
-__global__ void __launch_bounds__(kFFBlock) k_embed_pass2(Dev d, int st_clc, int row0)
+__global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_embed_pass2(Dev d, int st_clc, int row0)
 {
-    int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    constexpr int NV = 3;
+    __shared__ RowBuf<NV> sh[kFFWarps];
+    RowBuf<NV>& buf = sh[threadIdx.x >> 5];
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (i < d.natms) {
-        double4 xi = d.pos[i];
-        double dFi = d.rho[i];
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        int nn = d.nnb[i];
-        for (int k = lane; k < nn; k += 32) {
-            long long slot = (long long)i * d.maxnb + k;
-            double pi_ = d.pr[slot], pj_ = d.pr[d.maxp + slot];
-            if (pi_ != 0.0 || pj_ != 0.0) {
-                int j = d.nbr[slot];
-                double4 xj = d.pos[j];
-                double fpair = dFi * pi_ + d.rho[owner(d, j)] * pj_;
-                double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
-                fx += dx0 * fpair;
-                fy += dx1 * fpair;
-                fz += dx2 * fpair;
-                bool own_j = j < d.natms;
-                if (own_j) {
-                    double* fj = d.f + (size_t)j * 3;
-                    atomicAdd(fj + 0, -dx0 * fpair);
-                    atomicAdd(fj + 1, -dx1 * fpair);
-                    atomicAdd(fj + 2, -dx2 * fpair);
-                }
-                if (st_clc) {
-                    double wf = (own_j ? 1.0 : 0.5) * fpair;
-                    acc[1] -= wf * dx0 * dx0;
-                    acc[2] -= wf * dx1 * dx1;
-                    acc[3] -= wf * dx2 * dx2;
-                    acc[4] -= wf * dx1 * dx2;
-                    acc[5] -= wf * dx2 * dx0;
-                    acc[6] -= wf * dx0 * dx1;
-                }
+    for_pairs(d, [&](long long p, bool valid, int i) {
+        double f[3] = {0, 0, 0};
+        int row = -1;
+        if (valid) {
+            const int j = d.pair_j[p];
+            const double2 dr = __ldcs(reinterpret_cast<const double2*>(d.pr) + p);
+            if (dr.x != 0.0 || dr.y != 0.0) {
+                const double4 xi = d.pos[i], xj = d.pos[j];
+                const double fpair = d.rho[i] * dr.x + d.rho[owner(d, j)] * dr.y;
+                const double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
+                f[0] = -dx0 * fpair;
+                f[1] = -dx1 * fpair;
+                f[2] = -dx2 * fpair;
+                const bool own_j = j < d.natms;
+                if (own_j) row = j;
+                if (st_clc) add_virial(acc, (own_j ? 1.0 : 0.5) * fpair, dx0, dx1, dx2);
             }
         }
-        fx = warp_sum(fx);
-        fy = warp_sum(fy);
-        fz = warp_sum(fz);
-        if (lane == 0) {
-            atomicAdd(d.f + (size_t)i * 3 + 0, fx);
-            atomicAdd(d.f + (size_t)i * 3 + 1, fy);
-            atomicAdd(d.f + (size_t)i * 3 + 2, fz);
-        }
-    }
+        rows_put<3>(buf, f, i);
+        rows_scatter<3>(buf, row, [&](int r, int q, double x) { add_value(d, r, q, x); });
+        rows_runs<3>(buf, [&](int r, int q, double x) { add_value(d, r, q, -x); });
+    });
     block_partials<7>(acc, d.partial, row0 + blockIdx.x);
 }
 
 // Analytic FS pass 1 (ff_fs.cpp:424-527).
 template <bool kEnergyOnly>
-__global__ void __launch_bounds__(kFFBlock) k_fs_pass1(Dev d, int st_clc, int row0)
+__global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_fs_pass1(Dev d, int st_clc, int row0)
 {
-    int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    constexpr int NV = kEnergyOnly ? 1 : 4;
+    __shared__ RowBuf<NV> sh[kFFWarps];
+    RowBuf<NV>& buf = sh[threadIdx.x >> 5];
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (i < d.natms) {
-        double4 xi = d.pos[i];
-        int ti = d.type[i];
-        double rho_i = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-        int nn = d.nnb[i];
-        for (int k = lane; k < nn; k += 32) {
-            long long slot = (long long)i * d.maxnb + k;
-            int j = d.nbr[slot];
-            int tj = d.type[j];
-            int cs = comp_idx(ti, tj);
-            double pi_ = 0.0, pj_ = 0.0;
+    for_pairs(d, [&](long long p, bool valid, int i) {
+        double v[NV], rho_i = 0.0, pi_ = 0.0, pj_ = 0.0;
+#pragma unroll
+        for (int q = 0; q < NV; q++) v[q] = 0.0;
+        int row = -1;
+        if (valid) {
+            const int j = d.pair_j[p];
+            const int ti = d.type[i], tj = d.type[j];
+            const int cs = comp_idx(ti, tj);
             if (d.fs_chk[cs]) {
-                double4 xj = d.pos[j];
-                double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
-                double rsq = __dadd_rn(__dadd_rn(__dmul_rn(dx0, dx0), __dmul_rn(dx1, dx1)), __dmul_rn(dx2, dx2));
+                const double4 xi = d.pos[i], xj = d.pos[j];
+                const double dx0 = xi.x - xj.x, dx1 = xi.y - xj.y, dx2 = xi.z - xj.z;
+                const double rsq = __dadd_rn(__dadd_rn(__dmul_rn(dx0, dx0), __dmul_rn(dx1, dx1)), __dmul_rn(dx2, dx2));
                 if (rsq < d.fs_cut_sq[cs]) {
-                    double r = sqrt(rsq);
-                    double r_inv = 1.0 / r;
-                    bool own_j = j < d.natms;
-                    double w = own_j ? 1.0 : 0.5;
+                    const double r = sqrt(rsq);
+                    const double r_inv = 1.0 / r;
+                    const bool own_j = j < d.natms;
+                    const double w = own_j ? 1.0 : 0.5;
+                    if (own_j) row = j;
                     if (r < d.fs_cut_rho[cs]) {
-                        double dr_ = r - d.fs_cut_rho[cs];
-                        rho_i += dr_ * dr_ * (d.fst1[tj][ti] + d.fst2[tj][ti] * dr_);
-                        if (own_j) atomicAdd(&d.rho[j], dr_ * dr_ * (d.fst1[ti][tj] + d.fst2[ti][tj] * dr_));
+                        const double dr_ = r - d.fs_cut_rho[cs];
+                        rho_i = dr_ * dr_ * (d.fst1[tj][ti] + d.fst2[tj][ti] * dr_);
+                        v[NV - 1] = dr_ * dr_ * (d.fst1[ti][tj] + d.fst2[ti][tj] * dr_);
                         pi_ = -r_inv * dr_ * (d.fst1[tj][ti] + 1.5 * d.fst2[tj][ti] * dr_);
                         pj_ = -r_inv * dr_ * (d.fst1[ti][tj] + 1.5 * d.fst2[ti][tj] * dr_);
                     }
                     if (r < d.fs_cut_phi[cs]) {
-                        double dp = r - d.fs_cut_phi[cs];
-                        double poly = d.fsk1[cs] + d.fsk2[cs] * r + d.fsk3[cs] * rsq;
+                        const double dp = r - d.fs_cut_phi[cs];
+                        const double poly = d.fsk1[cs] + d.fsk2[cs] * r + d.fsk3[cs] * rsq;
                         acc[0] += w * (dp * dp * poly);
                         if (!kEnergyOnly) {
                             double pc = 2.0 * dp * poly + dp * dp * (d.fsk2[cs] + 2.0 * d.fsk3[cs] * r);
                             pc *= -r_inv;
-                            fx += dx0 * pc;
-                            fy += dx1 * pc;
-                            fz += dx2 * pc;
-                            if (own_j) {
-                                double* fj = d.f + (size_t)j * 3;
-                                atomicAdd(fj + 0, -dx0 * pc);
-                                atomicAdd(fj + 1, -dx1 * pc);
-                                atomicAdd(fj + 2, -dx2 * pc);
-                            }
-                            if (st_clc) {
-                                double wf = w * pc;
-                                acc[1] -= wf * dx0 * dx0;
-                                acc[2] -= wf * dx1 * dx1;
-                                acc[3] -= wf * dx2 * dx2;
-                                acc[4] -= wf * dx1 * dx2;
-                                acc[5] -= wf * dx2 * dx0;
-                                acc[6] -= wf * dx0 * dx1;
-                            }
+                            v[0] = -dx0 * pc;
+                            v[1 % NV] = -dx1 * pc;
+                            v[2 % NV] = -dx2 * pc;
+                            if (st_clc) add_virial(acc, w * pc, dx0, dx1, dx2);
                         }
                     }
                 }
             }
-            if (!kEnergyOnly) {
-                d.pr[slot] = pi_;
-                d.pr[d.maxp + slot] = pj_;
-            }
+            if (!kEnergyOnly) __stcs(reinterpret_cast<double2*>(d.pr) + p, make_double2(pi_, pj_));
         }
-        rho_i = warp_sum(rho_i);
-        if (!kEnergyOnly) {
-            fx = warp_sum(fx);
-            fy = warp_sum(fy);
-            fz = warp_sum(fz);
+        rows_put<NV>(buf, v, i);
+        rows_scatter<NV>(buf, row, [&](int r, int q, double x) { add_value(d, r, q + 4 - NV, x); });
+        {  // atom i's density is not atom j's
+            __syncwarp();
+            buf.v[(threadIdx.x & 31) * RowBuf<NV>::PITCH + NV - 1] = rho_i;
+            __syncwarp();
         }
-        if (lane == 0) {
-            atomicAdd(&d.rho[i], rho_i);
-            if (!kEnergyOnly) {
-                atomicAdd(d.f + (size_t)i * 3 + 0, fx);
-                atomicAdd(d.f + (size_t)i * 3 + 1, fy);
-                atomicAdd(d.f + (size_t)i * 3 + 2, fz);
-            }
-        }
-    }
+        rows_runs<NV>(buf, [&](int r, int q, double x) { add_value(d, r, q + 4 - NV, q + 4 - NV < 3 ? -x : x); });
+    });
     block_partials<7>(acc, d.partial, row0 + blockIdx.x);
 }
 
@@ -315,8 +269,9 @@ __global__ void __launch_bounds__(kFFBlock) k_fs_embed(Dev d, int row0)
 
 cudaError_t launch_eam_force(const Dev& d, int st_clc, int* nblocks_out, cudaStream_t st)
 {
-    int g1 = div_up((long long)d.natms * 32, kFFBlock), g2 = div_up(d.natms, kFFBlock);
-    k_eam_pass1<false><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
+    const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
+    if (d.nt == 1) k_eam_pass1<false, true><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
+    else k_eam_pass1<false, false><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
     k_eam_embed<false><<<g2, kFFBlock, 0, st>>>(d, g1);
     k_embed_pass2<<<g1, kFFBlock, 0, st>>>(d, st_clc, g1 + g2);
     *nblocks_out = 2 * g1 + g2;
@@ -325,8 +280,9 @@ cudaError_t launch_eam_force(const Dev& d, int st_clc, int* nblocks_out, cudaStr
 
 cudaError_t launch_eam_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 {
-    int g1 = div_up((long long)d.natms * 32, kFFBlock), g2 = div_up(d.natms, kFFBlock);
-    k_eam_pass1<true><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
+    const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
+    if (d.nt == 1) k_eam_pass1<true, true><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
+    else k_eam_pass1<true, false><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
     k_eam_embed<true><<<g2, kFFBlock, 0, st>>>(d, g1);
     *nblocks_out = g1 + g2;
     return cudaGetLastError();
@@ -334,7 +290,7 @@ cudaError_t launch_eam_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 
 cudaError_t launch_fs_force(const Dev& d, int st_clc, int* nblocks_out, cudaStream_t st)
 {
-    int g1 = div_up((long long)d.natms * 32, kFFBlock), g2 = div_up(d.natms, kFFBlock);
+    const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
     k_fs_pass1<false><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
     k_fs_embed<false><<<g2, kFFBlock, 0, st>>>(d, g1);
     k_embed_pass2<<<g1, kFFBlock, 0, st>>>(d, st_clc, g1 + g2);
@@ -344,7 +300,7 @@ cudaError_t launch_fs_force(const Dev& d, int st_clc, int* nblocks_out, cudaStre
 
 cudaError_t launch_fs_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 {
-    int g1 = div_up((long long)d.natms * 32, kFFBlock), g2 = div_up(d.natms, kFFBlock);
+    const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
     k_fs_pass1<true><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
     k_fs_embed<true><<<g2, kFFBlock, 0, st>>>(d, g1);
     *nblocks_out = g1 + g2;

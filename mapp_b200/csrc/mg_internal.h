@@ -94,7 +94,7 @@ struct Dev {
     double* a_in;
     double* g;
     // per-pair scratch
-    double* pr;    // EAM/FS: drhoi[maxp], drhoj[maxp]; DMD: 21 SoA blocks of maxp
+    double* pr;    // EAM/FS: {drhoi, drhoj} per pair; DMD: 21 SoA blocks of maxp
     long long maxp;
     // while act_on: the listed pairs whose stored densities and pair
     // energies are not all zero, as CSR over the owned sites (act_off[i],
@@ -130,9 +130,9 @@ struct Dev {
     // precision form: per ordered species pair (a,b) and knot, one 32-byte
     // sector {rho c0..c3 of slot b*nt+a, phi c0..c3 of slot COMP(a,b) (zero when a < b)}
     const float4* pkT;
-    // the plain form's copy of the same pairing in FP64: per ordered species
-    // pair (a,b) and knot one 64-byte record {rho c0..c3, phi c0..c3}, so the
-    // two knots a quadrature node needs share one cache line
+    // the same pairing in FP64, for the plain DMD form and EAM: per ordered
+    // species pair (a,b) and knot one 64-byte record {rho c0..c3, phi c0..c3},
+    // so the two knots a node needs share one cache line
     const double* pk64;
     // the precision form's table: the same splines resampled onto nrS =
     // kSplitKnots knots over [0, rc] (FP32 cubic Hermite pieces, float4

@@ -61,6 +61,95 @@ __device__ __forceinline__ double seg_sum(double v, const Seg& s)
     return v;
 }
 
+// Segments of a warp whose keys are sorted (equal keys in contiguous lanes,
+// padding lanes with key -1 at the end): boundaries from one shuffle and one
+// ballot instead of a match instruction.
+__device__ __forceinline__ Seg seg_sorted(int key)
+{
+    const int lane = threadIdx.x & 31;
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != key);
+    const unsigned upto = heads & (0xffffffffu >> (31 - lane));  // heads at or before this lane
+    const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
+    Seg sg;
+    sg.first = 31 - __clz(upto);
+    sg.last = after ? __ffs(after) - 2 : 31;
+    return sg;
+}
+
+// Sums of NV values per lane over a warp's pairs, through a shared-memory
+// buffer of the warp's own (RowBuf<NV>): rows_put writes the values (and each
+// lane's run key: the pairs' first site, equal keys in contiguous lanes, -1 for
+// none; only for rows_runs) and rows_scatter / rows_runs add them up, calling
+// put(row, q, x) for value q of row `row` (an atomic add).  One L1 data-stage
+// cycle goes to every shuffle and to every distinct line of a reduction:
+//  - rows_scatter: one row per lane.  NV reductions of 32 rows each would touch
+//    32 NV lines; with consecutive lanes on consecutive values of a row they
+//    touch about 32 + NV.
+//  - rows_runs: the sums of the runs of equal keys.  NV segmented shuffle sums of
+//    doubles take 10 NV shuffles; here a lane sums COLS consecutive pairs of one
+//    value and only the runs' ends are shuffled.
+template <int NV>
+struct RowBuf {
+    static constexpr int COLS = NV <= 2 ? 2 : (NV <= 4 ? 4 : 8);  // lanes side by side on a pair's values
+    static constexpr int PITCH = NV | 1;                          // odd: no bank conflicts
+    double v[32 * PITCH];
+    int key[32];
+};
+
+template <int NV>
+__device__ __forceinline__ void rows_put(RowBuf<NV>& b, const double (&v)[NV], int key)
+{
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NV; q++) b.v[lane * RowBuf<NV>::PITCH + q] = v[q];
+    b.key[lane] = key;
+    __syncwarp();
+}
+
+template <int NV, typename Put>
+__device__ __forceinline__ void rows_scatter(const RowBuf<NV>& b, int row, Put put)
+{
+    const int lane = threadIdx.x & 31;
+    if (!__any_sync(0xffffffffu, row >= 0)) return;
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        const int e = k * 32 + lane, src = e / NV, q = e - src * NV;
+        const int r = __shfl_sync(0xffffffffu, row, src);
+        const double x = b.v[src * RowBuf<NV>::PITCH + q];
+        if (r >= 0 && x != 0.0) put(r, q, x);
+    }
+}
+
+template <int NV, typename Put>
+__device__ __forceinline__ void rows_runs(const RowBuf<NV>& b, Put put)
+{
+    constexpr int COLS = RowBuf<NV>::COLS;
+    const int lane = threadIdx.x & 31, q = lane % COLS, p0 = (lane / COLS) * COLS;
+    int cur = b.key[p0];
+    double s = 0.0;
+#pragma unroll
+    for (int t = 0; t < COLS; t++) {
+        const int k = b.key[p0 + t];
+        if (k != cur) {
+            if (q < NV && cur >= 0 && s != 0.0) put(cur, q, s);
+            s = 0.0;
+            cur = k;
+        }
+        if (q < NV) s += b.v[(p0 + t) * RowBuf<NV>::PITCH + q];
+    }
+    // the ends of the COLS-pair stretches, joined over stretches of one run
+#pragma unroll
+    for (int o = COLS; o < 32; o <<= 1) {
+        const double t = __shfl_down_sync(0xffffffffu, s, o);
+        const int k = __shfl_down_sync(0xffffffffu, cur, o);
+        if (lane + o < 32 && k == cur) s += t;
+    }
+    const int prev = __shfl_up_sync(0xffffffffu, cur, COLS);
+    if (q < NV && cur >= 0 && (lane < COLS || prev != cur) && s != 0.0) put(cur, q, s);
+}
+
 // Batched form: is the cell of owned site i still being evaluated?
 __device__ __forceinline__ bool site_active(const Dev& d, int i)
 {
