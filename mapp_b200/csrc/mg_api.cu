@@ -1930,15 +1930,17 @@ int mg_mlp_train(mg_system* s, long long nsamples, int steps, int batch, double 
     fill_dev_scalars(s);
     CU(launch_mlp_labels(s->d, s->mlp.box, seed, n, X, Y, s->st));
     // output standardisation from the labels
-    std::vector<float> yh((size_t)n * 6);
-    CU(cudaMemcpyAsync(yh.data(), Y, yh.size() * sizeof(float), cudaMemcpyDeviceToHost, s->st));
+    const int rows = mlp_label_sum_rows(n);
+    CHK(ensure_partials(s, 2LL * rows));  // (12 of 16 doubles a row)
+    CU(launch_mlp_label_sums(Y, n, s->d.partial, s->st));
+    std::vector<double> sums((size_t)rows * 12);
+    CU(cudaMemcpyAsync(sums.data(), s->d.partial, sums.size() * sizeof(double), cudaMemcpyDeviceToHost, s->st));
     CU(cudaStreamSynchronize(s->st));
     for (int q = 0; q < 6; q++) {
         double m = 0, m2 = 0;
-        for (int k = 0; k < n; k++) {
-            double v = yh[(size_t)k * 6 + q];
-            m += v;
-            m2 += v * v;
+        for (int k = 0; k < rows; k++) {
+            m += sums[(size_t)k * 12 + q];
+            m2 += sums[(size_t)k * 12 + 6 + q];
         }
         m /= n;
         double var = m2 / n - m * m;

@@ -20,6 +20,7 @@
 // Species pairs: code 0 = (0,0), 1 = the unordered cross pair, 2 = (1,1); the
 // cross code uses one network for (0,1) and (1,0), which needs rho_AB =
 // rho_BA (true for the potentials this form is trained on).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -172,98 +173,330 @@ __global__ void k_mlp_labels(Dev d, MlpBox box, unsigned long long seed, int n, 
     y[5] = (float)(gda - base[5]);
 }
 
+// Sums of the labels and of their squares per output, one row of 12 doubles per
+// block (the caller adds the rows): the standardisation needs 96 bytes a block
+// instead of the whole label array on the host.
+__global__ void __launch_bounds__(256) k_mlp_label_sums(const float* __restrict__ Y, int n, double* __restrict__ out)
+{
+    __shared__ double sh[8][12];
+    double v[12];
+#pragma unroll
+    for (int q = 0; q < 12; q++) v[q] = 0.0;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const float2* y = reinterpret_cast<const float2*>(Y + 6 * k);
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            const float2 p = y[u];
+            v[2 * u] += (double)p.x;
+            v[2 * u + 1] += (double)p.y;
+            v[6 + 2 * u] += (double)p.x * (double)p.x;
+            v[7 + 2 * u] += (double)p.y * (double)p.y;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 12; q++) {
+        const double s = warp_sum(v[q]);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][q] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        double s = 0.0;
+        for (int w = 0; w < 8; w++) s += sh[w][threadIdx.x];
+        out[(size_t)blockIdx.x * 12 + threadIdx.x] = s;
+    }
+}
+
 // ---- one training step --------------------------------------------------------
 // CTA c takes rows idx = hash(seed, step, c*64 + r) % n of the training set,
 // or rows [c*64, c*64+64) of the given batch when `fixed` is set (gradient
 // checks).  Loss = mean over rows and outputs of the squared error of the
 // standardised outputs.
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_train(MlpState S, const float* __restrict__ X,
-                                                           const float* __restrict__ Y, int n, int batch,
-                                                           unsigned long long seed, int step, int fixed)
+//
+// What bounds it: latency -- a step has one 64-row tile per CTA (64 CTAs for
+// 4096 rows), ten dependent small products and a barrier between each.  So the
+// tile is spread over 16 warps that each own the same two 16x8 output tiles of
+// every 64x64 product (the pre-activations z stay in registers from the forward
+// to the backward pass and the activations are applied in the product's
+// epilogue), fragments come from padded rows by ldmatrix (conflict-free, the
+// transposed operands by its .trans form), and two further warps sum the bias
+// gradients beside the products.  With 4 warps, element loads of the fragments
+// (up to 8-way bank conflicts) and separate passes over z a step took 73 us; now
+// 14 us alone, and 14.4 us with its Adam kernel when the two overlap their starts
+// (83 before).  The products, their order of accumulation and every rounding are the
+// same, so the gradients are the same bits.
+constexpr int kTrainWarps = 16, kTrainThreads = (kTrainWarps + 2) * 32;
+constexpr int HP = H + 8;  // row pitch: 8 rows of 16 bytes fall into different banks
+
+struct TrainTile {
+    __nv_bfloat16 x[kRows][24], dy[kRows][24];
+    __nv_bfloat16 h[3][kRows][HP], dz[kRows][HP];
+    __nv_bfloat16 w1[16][HP], w2[H][HP], w3[H][HP], w4[H][8];
+    float zf[kRows][HP];
+    float y[kRows][8], tgt[kRows][8];
+    float b[3][H], b4[8], loss[4];
+};
+
+// Programmatic dependent launch: a step's two kernels are queued with
+// overlapping starts.  dep_start lets the next kernel's blocks be scheduled,
+// dep_wait returns when everything before this kernel in the stream is complete
+// and visible; what runs before it (the rows of a training tile) depends on
+// nothing the previous kernel writes.
+__device__ __forceinline__ void dep_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16* p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// Two neighbouring 16x8 tiles (columns n0 and n0 + 8) of A B over K in steps of
+// 16.  A is stored [m][k] (AT: [k][m]), B [k][n] (BN: [n][k]), pitches lda, ldb.
+template <bool AT, bool BN, int K>
+__device__ __forceinline__ void warp_gemm2(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int m0, int n0,
+                                           float (&c)[2][4])
+{
+    const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) c[j][q] = 0.f;
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        uint32_t a[4], b[4];
+        if (AT) ldsm4t(a, A + (k0 + (mat >> 1) * 8 + r) * lda + m0 + (mat & 1) * 8);
+        else ldsm4(a, A + (m0 + (mat & 1) * 8 + r) * lda + k0 + (mat >> 1) * 8);
+        if (BN) ldsm4(b, B + (n0 + (mat >> 1) * 8 + r) * ldb + k0 + (mat & 1) * 8);
+        else ldsm4t(b, B + (k0 + (mat & 1) * 8 + r) * ldb + n0 + (mat >> 1) * 8);
+        const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+        mma16816(c[0], a, b0);
+        mma16816(c[1], a, b1);
+    }
+}
+
+// one 16x8 tile with B stored [k][n] in rows of 8 (pitch ldb)
+template <bool AT, int K>
+__device__ __forceinline__ void warp_gemm8(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int m0, float (&c)[4])
+{
+    const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int q = 0; q < 4; q++) c[q] = 0.f;
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        uint32_t a[4], b[4];
+        ldsm4t(b, B + (k0 + mat * 8 + r) * ldb);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int k = k0 + 16 * u;
+            if (AT) ldsm4t(a, A + (k + (mat >> 1) * 8 + r) * lda + m0 + (mat & 1) * 8);
+            else ldsm4(a, A + (m0 + (mat & 1) * 8 + r) * lda + k + (mat >> 1) * 8);
+            const uint32_t bb[2] = {b[2 * u], b[2 * u + 1]};
+            mma16816(c, a, bb);
+        }
+    }
+}
+
+__device__ __forceinline__ void load_w(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int rows, int first, int k)
+{
+    // 16-byte piece k - first of a [rows][64] matrix, into rows of pitch HP
+    const int e = k - first;
+    if (e >= 0 && e < rows * 8)
+        *reinterpret_cast<uint4*>(dst + (e >> 3) * HP + (e & 7) * 8) = *reinterpret_cast<const uint4*>(src + e * 8);
+}
+
+__global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpState S, const float* __restrict__ X,
+                                                             const float* __restrict__ Y, int n, int batch,
+                                                             unsigned long long seed, int step, int fixed)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Tile& T = *reinterpret_cast<Tile*>(smem_raw);
-    __shared__ float tgt[kRows][8];
-    __shared__ float dsum[H];
-    __shared__ __nv_bfloat16 dy[kRows][16];
-    __shared__ __nv_bfloat16 dzb[kRows][H];
-    __shared__ float loss_sh;
-    load_weights(T, S.wbf, S.par);
-    if (threadIdx.x == 0) loss_sh = 0.f;
-    for (int r = threadIdx.x; r < kRows; r += blockDim.x) {
-        long long row = (long long)blockIdx.x * kRows + r;
-        long long idx = fixed ? row : (long long)(mix64(seed ^ (0x10000000000ull * (unsigned long long)(step + 1)) ^
-                                                        (unsigned long long)row) %
-                                                  (unsigned long long)n);
-        float in[4];
-        net_inputs(S.box, X[4 * idx], X[4 * idx + 1], X[4 * idx + 2], (int)X[4 * idx + 3], in);
-        for (int k = 0; k < 16; k++) T.x[r][k] = __float2bfloat16(k < 4 ? in[k] : 0.f);
-        for (int q = 0; q < 8; q++) tgt[r][q] = q < 6 ? (Y[6 * idx + q] - S.out_mean[q]) / S.out_scale[q] : 0.f;
+    TrainTile& T = *reinterpret_cast<TrainTile*>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    dep_start();
+    // 8 threads per row: one takes the inputs, six a target each
+    if (tid < kRows * 8) {
+        const int r = tid >> 3, part = tid & 7;
+        const long long row = (long long)blockIdx.x * kRows + r;
+        const long long idx = fixed ? row : (long long)(mix64(seed ^ (0x10000000000ull * (unsigned long long)(step + 1)) ^
+                                                              (unsigned long long)row) %
+                                                        (unsigned long long)n);
+        if (part == 0) {
+            float in[4];
+            net_inputs(S.box, X[4 * idx], X[4 * idx + 1], X[4 * idx + 2], (int)X[4 * idx + 3], in);
+            uint4* xr = reinterpret_cast<uint4*>(T.x[r]);
+            xr[0] = make_uint4(pack2f(in[0], in[1]), pack2f(in[2], in[3]), 0u, 0u);
+            xr[1] = make_uint4(0u, 0u, 0u, 0u);
+        } else if (part < 7) {
+            const int q = part - 1;
+            T.tgt[r][q] = (Y[6 * idx + q] - S.out_mean[q]) / S.out_scale[q];
+        } else
+            reinterpret_cast<uint4*>(T.dy[r])[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    dep_wait();  // the previous step's weights
+    for (int k = tid; k < 1216; k += kTrainThreads) {
+        load_w(&T.w1[0][0], S.wbf + OW1, 16, 0, k);
+        load_w(&T.w2[0][0], S.wbf + OW2, H, 128, k);
+        load_w(&T.w3[0][0], S.wbf + OW3, H, 640, k);
+        if (k >= 1152) reinterpret_cast<uint4*>(&T.w4[0][0])[k - 1152] = reinterpret_cast<const uint4*>(S.wbf + OW4)[k - 1152];
+    }
+    if (tid < H) {
+        T.b[0][tid] = S.par[OB1 + tid];
+        T.b[1][tid] = S.par[OB2 + tid];
+        T.b[2][tid] = S.par[OB3 + tid];
+        if (tid < 8) T.b4[tid] = S.par[OB4 + tid];
     }
     __syncthreads();
-    forward(T, S.act);
+    const bool gw = warp < kTrainWarps;
+    const int m0 = (warp >> 2) * 16, n0 = (warp & 3) * 16;
+    float z[3][2][4], c[2][4];
+    // forward: z = h W + b in registers, h in shared memory
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+        if (gw) {
+            if (l == 0) warp_gemm2<false, false, 16>(&T.x[0][0], 24, &T.w1[0][0], HP, m0, n0, c);
+            else warp_gemm2<false, false, H>(&T.h[l - 1][0][0], HP, l == 1 ? &T.w2[0][0] : &T.w3[0][0], HP, m0, n0, c);
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int col = n0 + 8 * j + 2 * t;
+#pragma unroll
+                for (int q = 0; q < 4; q++) z[l][j][q] = c[j][q] + T.b[l][col + (q & 1)];
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    *reinterpret_cast<uint32_t*>(&T.h[l][m0 + g + 8 * u][col]) =
+                        pack2f(act_rt(S.act, col, z[l][j][2 * u]), act_rt(S.act, col + 1, z[l][j][2 * u + 1]));
+            }
+        }
+        __syncthreads();
+    }
     float* gp = S.gpart + (size_t)blockIdx.x * NPART;
     const float inv = 2.0f / ((float)batch * 6.0f);
-    // dL/dy
-    for (int e = threadIdx.x; e < kRows * 16; e += blockDim.x) {
-        int r = e / 16, q = e % 16;
-        float v = 0.f;
-        if (q < 6) {
-            float diff = T.y[r][q] - tgt[r][q];
-            v = inv * diff;
-            atomicAdd(&loss_sh, diff * diff / ((float)batch * 6.0f));
+    // output layer, dL/dy (BF16 for the products, FP32 for the bias gradient), loss
+    if (warp < 4) {
+        float o[4], sum = 0.f;
+        warp_gemm8<false, H>(&T.h[2][0][0], HP, &T.w4[0][0], 8, warp * 16, o);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int r = warp * 16 + g + 8 * u;
+            float v[2] = {0.f, 0.f};
+            if (t < 3) {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float diff = o[2 * u + e] + T.b4[2 * t + e] - T.tgt[r][2 * t + e];
+                    v[e] = inv * diff;
+                    sum += diff * diff / ((float)batch * 6.0f);
+                }
+            }
+            *reinterpret_cast<uint32_t*>(&T.dy[r][2 * t]) = pack2f(v[0], v[1]);
+            *reinterpret_cast<float2*>(&T.y[r][2 * t]) = make_float2(v[0], v[1]);
         }
-        dy[r][q] = __float2bfloat16(v);
-        if (q < 8) T.y[r][q] = q < 6 ? v : 0.f;  // keep FP32 dL/dy for the bias gradient
+        sum = warp_sumf(sum);
+        if (lane == 0) T.loss[warp] = sum;
     }
     __syncthreads();
-    // layer 4: dW4 = h3^T dy, db4 = sum dy, dh3 = dy W4^T
-    cta_gemm<H, 8, kRows>([&](int m, int k) { return T.h[2][k][m]; }, [&](int k, int n2) { return dy[k][n2]; },
-                          [&](int m, int n2, float v) { gp[OW4 + m * 8 + n2] = v; });
-    if (threadIdx.x < 8) {
+    // layer 4: dh3 = dy W4^T (its K of 16 is 8 outputs and zeros); dW4 = h3^T dy, db4 = sum dy
+    auto put_dz = [&]() {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int col = n0 + 8 * j + 2 * t;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const float v0 = c[j][2 * u], v1 = c[j][2 * u + 1];
+                *reinterpret_cast<float2*>(&T.zf[m0 + g + 8 * u][col]) = make_float2(v0, v1);
+                *reinterpret_cast<uint32_t*>(&T.dz[m0 + g + 8 * u][col]) = pack2f(v0, v1);
+            }
+        }
+    };
+    auto times_dact = [&](int l) {
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                c[j][q] = c[j][q] * dact_rt(S.act, n0 + 8 * j + 2 * t + (q & 1), z[l][j][q]);
+    };
+    if (gw) {
+        uint32_t a[4], b[4];
+        const int mat = lane >> 3, r = lane & 7;
+        ldsm4(a, &T.dy[m0 + (mat & 1) * 8 + r][(mat >> 1) * 8]);
+        ldsm4(b, &T.w4[n0 + (mat & 1) * 8 + r][0]);
+        const uint32_t b0[2] = {b[0], 0u}, b1[2] = {b[1], 0u};
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) c[j][q] = 0.f;
+        mma16816(c[0], a, b0);
+        mma16816(c[1], a, b1);
+        times_dact(2);
+        put_dz();
+        if (warp < 4) {
+            float o[4];
+            warp_gemm8<true, kRows>(&T.h[2][0][0], HP, &T.dy[0][0], 24, warp * 16, o);
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                *reinterpret_cast<float2*>(&gp[OW4 + (warp * 16 + g + 8 * u) * 8 + 2 * t]) = make_float2(o[2 * u], o[2 * u + 1]);
+        }
+    } else if (warp == kTrainWarps && lane < 8) {
         float s = 0.f;
-        for (int r = 0; r < kRows; r++) s += T.y[r][threadIdx.x];
-        gp[OB4 + threadIdx.x] = s;
+#pragma unroll 16
+        for (int r = 0; r < kRows; r++) s += T.y[r][lane];
+        gp[OB4 + lane] = s;
     }
-    cta_gemm<kRows, H, 16>([&](int m, int k) { return dy[m][k]; },
-                           [&](int k, int n2) { return k < 8 ? T.w4[n2][k] : __float2bfloat16(0.f); },
-                           [&](int m, int n2, float v) { T.z[2][m][n2] = v * dact_rt(S.act, n2, T.z[2][m][n2]); });
     __syncthreads();
-    // layers 3, 2, 1: z[l] now holds dL/dz_l
+    // layers 3, 2, 1: zf and dz hold dL/dz_l
+#pragma unroll
     for (int l = 2; l >= 0; l--) {
-        for (int e = threadIdx.x; e < kRows * H; e += blockDim.x) (&dzb[0][0])[e] = __float2bfloat16((&T.z[l][0][0])[e]);
-        for (int c = threadIdx.x; c < H; c += blockDim.x) {
-            float s = 0.f;
-            for (int r = 0; r < kRows; r++) s += T.z[l][r][c];
-            dsum[c] = s;
-        }
-        __syncthreads();
         const int ow = l == 2 ? OW3 : (l == 1 ? OW2 : OW1), ob = l == 2 ? OB3 : (l == 1 ? OB2 : OB1);
-        for (int c = threadIdx.x; c < H; c += blockDim.x) gp[ob + c] = dsum[c];
-        if (l > 0) {
-            cta_gemm<H, H, kRows>([&](int m, int k) { return T.h[l - 1][k][m]; }, [&](int k, int n2) { return dzb[k][n2]; },
-                                  [&](int m, int n2, float v) { gp[ow + m * H + n2] = v; });
-            const __nv_bfloat16(*W)[H] = l == 2 ? T.w3 : T.w2;
-            cta_gemm<kRows, H, H>([&](int m, int k) { return dzb[m][k]; }, [&](int k, int n2) { return W[n2][k]; },
-                                  [&](int m, int n2, float v) { T.z[l - 1][m][n2] = v * dact_rt(S.act, n2, T.z[l - 1][m][n2]); });
+        if (gw) {
+            if (l > 0 || warp < 4) {
+                float w[2][4];
+                if (l > 0) warp_gemm2<true, false, kRows>(&T.h[l > 0 ? l - 1 : 0][0][0], HP, &T.dz[0][0], HP, m0, n0, w);
+                else warp_gemm2<true, false, kRows>(&T.x[0][0], 24, &T.dz[0][0], HP, 0, n0, w);
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++)
+                        *reinterpret_cast<float2*>(&gp[ow + ((l > 0 ? m0 : 0) + g + 8 * u) * H + n0 + 8 * j + 2 * t]) =
+                            make_float2(w[j][2 * u], w[j][2 * u + 1]);
+            }
+            if (l > 0) {
+                warp_gemm2<false, true, H>(&T.dz[0][0], HP, l == 2 ? &T.w3[0][0] : &T.w2[0][0], HP, m0, n0, c);
+                times_dact(l - 1);
+            }
         } else {
-            cta_gemm<16, H, kRows>([&](int m, int k) { return T.x[k][m]; }, [&](int k, int n2) { return dzb[k][n2]; },
-                                   [&](int m, int n2, float v) { gp[OW1 + m * H + n2] = v; });
+            const int col = tid - kTrainWarps * 32;
+            float s = 0.f;
+#pragma unroll 16
+            for (int r = 0; r < kRows; r++) s += T.zf[r][col];
+            gp[ob + col] = s;
         }
-        __syncthreads();
+        if (l > 0) {
+            __syncthreads();
+            if (gw) put_dz();
+            __syncthreads();
+        }
     }
-    if (threadIdx.x == 0) gp[OLOSS] = loss_sh;
+    if (tid == 0) gp[OLOSS] = (T.loss[0] + T.loss[1]) + (T.loss[2] + T.loss[3]);
 }
 
 // Sum of the per-CTA partial gradients; Adam (Kingma & Ba 2015) with a cosine
 // learning rate; BF16 copy of the weights.  With lr == 0 only the summed
-// gradient is written (gradient checks).
-__global__ void k_mlp_adam(MlpState S, int nblocks, int step, int total_steps, float lr0, float* __restrict__ grad_out,
+// gradient is written (gradient checks).  Small blocks, so that the reads of the
+// partials spread over all SMs.
+constexpr int kAdamThreads = 64;
+__global__ void __launch_bounds__(kAdamThreads) k_mlp_adam(MlpState S, int nblocks, int step, int total_steps, float lr0, float* __restrict__ grad_out,
                            float* __restrict__ loss_hist)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
+    dep_start();
     if (p > NPARAM) return;
+    dep_wait();  // this step's partial gradients
     float g = 0.f;
+#pragma unroll 16
     for (int c = 0; c < nblocks; c++) g += S.gpart[(size_t)c * NPART + p];
     if (p == NPARAM) {
         if (loss_hist) loss_hist[step] = g;
@@ -324,21 +557,41 @@ cudaError_t launch_mlp_labels(const Dev& d, const MlpBox& box, unsigned long lon
     return cudaGetLastError();
 }
 
+int mlp_label_sum_rows(int n) { return std::min(div_up(n, 256), 2 * num_sms()); }
+
+cudaError_t launch_mlp_label_sums(const float* Y, int n, double* out, cudaStream_t st)
+{
+    k_mlp_label_sums<<<mlp_label_sum_rows(n), 256, 0, st>>>(Y, n, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_mlp_train_step(const MlpState& S, const float* X, const float* Y, int n, int batch,
                                   unsigned long long seed, int step, int total, float lr, int fixed, float* grad_out,
                                   float* loss_hist, cudaStream_t st)
 {
-    static bool attr = false;
-    size_t sm = sizeof(Tile);
-    if (!attr) {
-        cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaFuncSetAttribute(k_mlp_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        attr = true;
+    constexpr size_t sm = sizeof(TrainTile);
+    if (step == 0 || fixed) {
+        const cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
     }
     int nb = batch / kRows;
-    k_mlp_train<<<nb, kMlpThreads, sm, st>>>(S, X, Y, n, batch, seed, step, fixed);
-    k_mlp_adam<<<div_up(NPARAM + 1, 256), 256, 0, st>>>(S, nb, step, total, lr, grad_out, loss_hist);
-    return cudaGetLastError();
+    cudaLaunchAttribute dep;
+    dep.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    dep.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kTrainThreads);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cfg.attrs = &dep;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_mlp_train, S, X, Y, n, batch, seed, step, fixed);
+    if (e != cudaSuccess) return e;
+    cfg.gridDim = dim3(div_up(NPARAM + 1, kAdamThreads));
+    cfg.blockDim = dim3(kAdamThreads);
+    cfg.dynamicSmemBytes = 0;
+    e = cudaLaunchKernelEx(&cfg, k_mlp_adam, S, nb, step, total, lr, grad_out, loss_hist);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_mlp_eval(const MlpState& S, const float* X, int n, float* Y, cudaStream_t st)

@@ -26,7 +26,8 @@ namespace mlp {
 constexpr int H = 64;  // hidden width
 // parameter offsets of the FP32 master vector (W stored [in][out])
 constexpr int OW1 = 0, OB1 = OW1 + 16 * H, OW2 = OB1 + H, OB2 = OW2 + H * H, OW3 = OB2 + H, OB3 = OW3 + H * H,
-              OW4 = OB3 + H, OB4 = OW4 + H * 8, NPARAM = OB4 + 8, OLOSS = NPARAM, NPART = NPARAM + 1;
+              OW4 = OB3 + H, OB4 = OW4 + H * 8, NPARAM = OB4 + 8, OLOSS = NPARAM,
+              NPART = NPARAM + 4;  // (16-byte rows)
 
 // Activation silu_p(z) = z * sigma_p(z), with sigma_p a polynomial stand-in for
 // the logistic function that runs on the FP32 FMA pipe (no transcendental
