@@ -17,7 +17,7 @@ BUILD = os.path.join(HERE, "_build")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 SOURCES = ["mg_api.cu", "mg_atoms.cu", "mg_eam.cu", "mg_dmd.cu", "mg_dmd32.cu", "mg_mlp.cu", "mg_mlp_tc.cu", "mg_noalloc.cu", "mg_batch.cu", "mg_cfg.cu", "mg_md.cu", "mg_clock.cu"]
-HEADERS = ["mg_internal.h", "mg_reduce.cuh", "mg_dmd_common.cuh", "mg_mlp_common.cuh", "mg_split.cuh"]
+HEADERS = ["mg_internal.h", "mg_reduce.cuh", "mg_dmd_common.cuh", "mg_mlp_common.cuh", "mg_split.cuh", "mg_launch.cuh"]
 
 # a C++ client of the C ABI (the end-to-end measurement of bench.py)
 CLIENT_SRC = os.path.join(HERE, "client", "mapp_e2e.cpp")

@@ -1501,14 +1501,13 @@ int mg_ff_force_calc(mg_system* s, int st_clc, double* f, double* en_st)
     // the precision form's first kernel zeroes f and E itself
     const bool f32 = s->dmd && s->form == MG_FORM_FP32;
     // (and the plain DMD form's embedding kernel writes f's first terms)
-    if (!f32 && !(s->dmd && s->form == MG_FORM_FP64))
-        CU(cudaMemsetAsync(d.f, 0, (size_t)s->natms * s->x_dim * sizeof(double), s->st));
+    const size_t nf = f32 || (s->dmd && s->form == MG_FORM_FP64) ? 0 : (size_t)s->natms * s->x_dim;
     int rows = 0;
     if (s->style == STYLE_EAM || s->style == STYLE_FS) {
-        CU(cudaMemsetAsync(d.rho, 0, (size_t)s->natms * sizeof(double), s->st));
+        CU(launch_zero(d.f, nf, d.rho, (size_t)s->natms, s->st));
         CU(s->style == STYLE_EAM ? launch_eam_force(d, st_clc, &rows, s->st) : launch_fs_force(d, st_clc, &rows, s->st));
     } else {
-        if (!f32) CU(cudaMemsetAsync(d.E, 0, (size_t)s->natms * s->nt * sizeof(double), s->st));
+        if (!f32) CU(launch_zero(d.f, nf, d.E, (size_t)s->natms * s->nt, s->st));
         if (f32) {
             CU(launch_dmd_force_f32(d, st_clc, &rows, s->st, evk));
             s->prf_stale = true;
@@ -1587,10 +1586,10 @@ int mg_ff_energy_calc(mg_system* s, double* energy)
     CHK(timed_begin(s));
     int rows = 0;
     if (s->style == STYLE_EAM || s->style == STYLE_FS) {
-        CU(cudaMemsetAsync(d.rho, 0, (size_t)s->natms * sizeof(double), s->st));
+        CU(launch_zero(d.rho, (size_t)s->natms, nullptr, 0, s->st));
         CU(s->style == STYLE_EAM ? launch_eam_energy(d, &rows, s->st) : launch_fs_energy(d, &rows, s->st));
     } else {
-        CU(cudaMemsetAsync(d.E, 0, (size_t)s->natms * s->nt * sizeof(double), s->st));
+        CU(launch_zero(d.E, (size_t)s->natms * s->nt, nullptr, 0, s->st));
         CU(launch_dmd_energy(d, &rows, s->st));
     }
     CU(launch_reduce_partials(d, rows, 1, s->red_out, s->st));
@@ -1643,8 +1642,7 @@ int mg_ff_c_d_calc(mg_system* s, double* c_d)
     size_t bytes = (size_t)s->natms * s->nt * sizeof(double);
     CHK(timed_begin(s));
     CHK(ensure_pair_values(s));
-    CU(cudaMemsetAsync(d.E, 0, bytes, s->st));
-    CU(cudaMemsetAsync(d.c_d, 0, bytes, s->st));
+    CU(launch_zero(d.E, bytes / sizeof(double), d.c_d, bytes / sizeof(double), s->st));
     CU(launch_dmd_cdot(d, s->st));
     CHK(timed_end(s));
     CHK(copy_out(s, c_d, d.c_d, bytes));
@@ -1672,7 +1670,7 @@ int mg_ff_calc_g(mg_system* s, int chk, double alpha, const double* a, double* g
     CU(cudaMemcpyAsync(d.a_in, a, bytes, is_device_ptr(a) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s->st));
     CHK(timed_begin(s));
     CHK(ensure_pair_values(s));
-    CU(cudaMemsetAsync(d.E, 0, bytes, s->st));
+    CU(launch_zero(d.E, bytes / sizeof(double), nullptr, 0, s->st));
     int rows = 0;
     CU(launch_dmd_calc_g(d, chk, alpha, &rows, s->st));
     CHK(copy_out_side(s, g, d.g, bytes));
@@ -2075,8 +2073,7 @@ int mg::system_enqueue_force(mg_system* s, int st_clc, int zero, int* rows)
         return fail(MG_ERR_UNSUPPORTED, "the device MD loop drives EAM / FS force fields");
     Dev& d = s->d;
     if (zero) {
-        CU(cudaMemsetAsync(d.f, 0, (size_t)s->natms * s->x_dim * sizeof(double), s->st));
-        CU(cudaMemsetAsync(d.rho, 0, (size_t)s->natms * sizeof(double), s->st));
+        CU(launch_zero(d.f, (size_t)s->natms * s->x_dim, d.rho, (size_t)s->natms, s->st));
     }
     CU(s->style == STYLE_EAM ? launch_eam_force(d, st_clc, rows, s->st) : launch_fs_force(d, st_clc, rows, s->st));
     return MG_OK;
@@ -2088,7 +2085,7 @@ int mg::system_enqueue_calc_g(mg_system* s, int chk, double alpha, int* rows)
     if (!s->crd_built) return fail(MG_ERR_STATE, "create_2nd_neigh_lst must run before calc_g");
     CHK(ensure_pair_values(s));
     Dev& d = s->d;
-    CU(cudaMemsetAsync(d.E, 0, (size_t)s->natms * s->nt * sizeof(double), s->st));
+    CU(launch_zero(d.E, (size_t)s->natms * s->nt, nullptr, 0, s->st));
     CU(launch_dmd_calc_g(d, chk, alpha, rows, s->st));
     CU(launch_reduce_partials(d, *rows, 1, s->red_out, s->st));
     return MG_OK;
@@ -2101,7 +2098,7 @@ int mg::system_enqueue_calc_g_dev(mg_system* s, const int* chk_dev, const double
     Dev d = s->d;
     d.g_chk = chk_dev;
     d.g_alpha = alpha_dev;
-    CU(cudaMemsetAsync(d.E, 0, (size_t)s->natms * s->nt * sizeof(double), s->st));
+    CU(launch_zero(d.E, (size_t)s->natms * s->nt, nullptr, 0, s->st));
     CU(launch_dmd_calc_g(d, 0, 0.0, rows, s->st));
     CU(launch_reduce_partials(d, *rows, 1, s->red_out, s->st));
     return MG_OK;
@@ -2146,8 +2143,7 @@ int mg::system_enqueue_c_d(mg_system* s)
     CHK(ensure_pair_values(s));
     Dev& d = s->d;
     size_t bytes = (size_t)s->natms * s->nt * sizeof(double);
-    CU(cudaMemsetAsync(d.E, 0, bytes, s->st));
-    CU(cudaMemsetAsync(d.c_d, 0, bytes, s->st));
+    CU(launch_zero(d.E, bytes / sizeof(double), d.c_d, bytes / sizeof(double), s->st));
     CU(launch_dmd_cdot(d, s->st));
     return MG_OK;
 }

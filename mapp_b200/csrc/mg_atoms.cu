@@ -11,6 +11,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "mg_internal.h"
+#include "mg_launch.cuh"
 
 namespace mg {
 
@@ -33,6 +34,7 @@ __device__ __forceinline__ void set3(double4& p, int k, double v)
 
 __global__ void k_split_x(Dev d, const double* __restrict__ x, int frac)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.natms) return;
     const double* p = x + (size_t)i * d.x_dim;
@@ -45,6 +47,7 @@ __global__ void k_split_x(Dev d, const double* __restrict__ x, int frac)
 // Atoms::x2s for owned atoms, including the wrap loops into [0, 1).
 __global__ void k_x2s(Dev d)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.natms) return;
     double4 p = d.pos[i];
@@ -98,6 +101,7 @@ __global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* __
                                                        int* __restrict__ ticket, int* __restrict__ ticket_next, int cap,
                                                        int dim, int dir, int next_mode)
 {
+    dep_sync();
     __shared__ int s_tile, s_excl;
     __shared__ int s_warp[kBlock / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -227,6 +231,7 @@ __global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* __
 
 __global__ void k_ghost_ctl_init(Dev d, GhostCtl* c)
 {
+    dep_sync();
     GhostCtl o;
     o.lo = 0;
     o.hi = d.natms;
@@ -247,6 +252,7 @@ __device__ __forceinline__ int nall_of(const Dev& d, const GhostCtl* gc, int cap
 // atoms per bin.
 __global__ void k_bin_s2x(Dev d, const GhostCtl* __restrict__ gc, int cap)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nall_of(d, gc, cap)) return;
     double4 s = d.sfr[i];
@@ -276,6 +282,7 @@ __device__ __forceinline__ int unpack_type(double w) { return (int)(__double_as_
 
 __global__ void k_cell_fill(Dev d, int* __restrict__ cursor, const GhostCtl* __restrict__ gc, int cap)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nall_of(d, gc, cap)) return;
     int b = d.bin[i];
@@ -290,6 +297,7 @@ __global__ void k_cell_fill(Dev d, int* __restrict__ cursor, const GhostCtl* __r
 // and a ballot compacts the accepted j (> i, rsq < cut_sk_sq) into the list.
 __global__ void __launch_bounds__(kBlock) k_neigh(Dev d)
 {
+    dep_sync();
     int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (i >= d.natms) return;
@@ -349,6 +357,7 @@ __global__ void __launch_bounds__(kBlock) k_neigh(Dev d)
 // Compact CSR copy of the half list: pair p = poff[i] + k is (i, nbr[i][k]).
 __global__ void __launch_bounds__(kBlock) k_pairs_compact(Dev d)
 {
+    dep_sync();
     int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (i >= d.natms) return;
@@ -361,6 +370,7 @@ __global__ void __launch_bounds__(kBlock) k_pairs_compact(Dev d)
 
 __global__ void k_store_x0(Dev d)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.natms) d.pos0[i] = d.pos[i];
 }
@@ -374,6 +384,7 @@ __global__ void k_store_x0(Dev d)
 // caller makes new for every call, to *flag, so the word needs no reset.
 __global__ void k_update_x(Dev d, const double* __restrict__ x, double sq_skin, int* __restrict__ flag, int gen)
 {
+    dep_sync();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < d.natms) {
         const double* p = x + (size_t)k * d.x_dim;
@@ -394,14 +405,26 @@ __global__ void k_update_x(Dev d, const double* __restrict__ x, double sq_skin, 
 
 __global__ void k_refresh_c(Dev d)
 {
+    dep_sync();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= d.nph) return;
     int g = d.natms + k, r = d.root[g];
     for (int a = 0; a < d.nt; a++) d.c[(size_t)g * d.nt + a] = d.c[(size_t)r * d.nt + a];
 }
 
+// a[0..na) and b[0..nb) to zero: a kernel rather than a memset, so that the
+// first pair pass behind it can be queued with an overlapping start
+__global__ void __launch_bounds__(kBlock) k_zero(double* __restrict__ a, size_t na, double* __restrict__ b, size_t nb)
+{
+    dep_sync();
+    const size_t k = (size_t)blockIdx.x * kBlock + threadIdx.x;
+    if (k < na) a[k] = 0.0;
+    else if (k - na < nb) b[k - na] = 0.0;
+}
+
 __global__ void k_merge_x(Dev d, double* __restrict__ x, int first, int count)
 {
+    dep_sync();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     int i = first + k;
@@ -419,6 +442,7 @@ __global__ void k_merge_x(Dev d, double* __restrict__ x, int first, int count)
 __global__ void __launch_bounds__(1024) k_reduce_partials(const double* __restrict__ partial, int nblocks, int nvals,
                                                          double* __restrict__ out)
 {
+    dep_sync();
     __shared__ double sh[32][8];
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
@@ -461,19 +485,19 @@ int num_sms()
 
 cudaError_t launch_split_x(const Dev& d, const double* x_aos, int frac, cudaStream_t st)
 {
-    if (d.natms) k_split_x<<<div_up(d.natms, kBlock), kBlock, 0, st>>>(d, x_aos, frac);
+    if (d.natms) launch_dep(k_split_x, div_up(d.natms, kBlock), kBlock, 0, st, d, x_aos, frac);
     return cudaGetLastError();
 }
 
 cudaError_t launch_x2s(const Dev& d, cudaStream_t st)
 {
-    if (d.natms) k_x2s<<<div_up(d.natms, kBlock), kBlock, 0, st>>>(d);
+    if (d.natms) launch_dep(k_x2s, div_up(d.natms, kBlock), kBlock, 0, st, d);
     return cudaGetLastError();
 }
 
 cudaError_t launch_ghost_init(const Dev& d, GhostCtl* ctl, cudaStream_t st)
 {
-    k_ghost_ctl_init<<<1, 1, 0, st>>>(d, ctl);
+    launch_dep(k_ghost_ctl_init, 1, 1, 0, st, d, ctl);
     return cudaGetLastError();
 }
 
@@ -482,7 +506,7 @@ int ghost_tiles(int cap) { return (cap + kGhostTile - 1) / kGhostTile; }
 cudaError_t launch_ghost_pass(const Dev& d, const GhostCtl* ctl, GhostCtl* next, unsigned* tiles, unsigned* tiles_next,
                               int* ticket, int* ticket_next, int cap, int dim, int dir, int next_mode, cudaStream_t st)
 {
-    k_ghost_pass<<<std::max(ghost_tiles(cap), 1), kBlock, 0, st>>>(d, ctl, next, tiles, tiles_next, ticket,
+    launch_dep(k_ghost_pass, std::max(ghost_tiles(cap), 1), kBlock, 0, st, d, ctl, next, tiles, tiles_next, ticket,
                                                                    ticket_next, cap, dim, dir, next_mode);
     return cudaGetLastError();
 }
@@ -490,57 +514,63 @@ cudaError_t launch_ghost_pass(const Dev& d, const GhostCtl* ctl, GhostCtl* next,
 cudaError_t launch_bin_and_s2x(const Dev& d, const GhostCtl* gc, int cap, cudaStream_t st)
 {
     const int n = gc ? cap : d.nall;
-    if (n) k_bin_s2x<<<div_up(n, kBlock), kBlock, 0, st>>>(d, gc, cap);
+    if (n) launch_dep(k_bin_s2x, div_up(n, kBlock), kBlock, 0, st, d, gc, cap);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cell_fill(const Dev& d, int* cursor, const GhostCtl* gc, int cap, cudaStream_t st)
 {
     const int n = gc ? cap : d.nall;
-    if (n) k_cell_fill<<<div_up(n, kBlock), kBlock, 0, st>>>(d, cursor, gc, cap);
+    if (n) launch_dep(k_cell_fill, div_up(n, kBlock), kBlock, 0, st, d, cursor, gc, cap);
     return cudaGetLastError();
 }
 
 cudaError_t launch_neigh(const Dev& d, cudaStream_t st)
 {
-    if (d.natms) k_neigh<<<div_up((long long)d.natms * 32, kBlock), kBlock, 0, st>>>(d);
+    if (d.natms) launch_dep(k_neigh, div_up((long long)d.natms * 32, kBlock), kBlock, 0, st, d);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pairs_compact(const Dev& d, cudaStream_t st)
 {
-    if (d.natms) k_pairs_compact<<<div_up((long long)d.natms * 32, kBlock), kBlock, 0, st>>>(d);
+    if (d.natms) launch_dep(k_pairs_compact, div_up((long long)d.natms * 32, kBlock), kBlock, 0, st, d);
     return cudaGetLastError();
 }
 
 cudaError_t launch_store_x0(const Dev& d, cudaStream_t st)
 {
-    if (d.natms) k_store_x0<<<div_up(d.natms, kBlock), kBlock, 0, st>>>(d);
+    if (d.natms) launch_dep(k_store_x0, div_up(d.natms, kBlock), kBlock, 0, st, d);
     return cudaGetLastError();
 }
 
 cudaError_t launch_update_x(const Dev& d, const double* x_aos, double sq_skin, int* flag, int gen, cudaStream_t st)
 {
     const int n = d.natms + d.nph;
-    if (n) k_update_x<<<div_up(n, kBlock), kBlock, 0, st>>>(d, x_aos, sq_skin, flag, gen);
+    if (n) launch_dep(k_update_x, div_up(n, kBlock), kBlock, 0, st, d, x_aos, sq_skin, flag, gen);
     return cudaGetLastError();
 }
 
 cudaError_t launch_refresh_c(const Dev& d, cudaStream_t st)
 {
-    if (d.nph && d.c) k_refresh_c<<<div_up(d.nph, kBlock), kBlock, 0, st>>>(d);
+    if (d.nph && d.c) launch_dep(k_refresh_c, div_up(d.nph, kBlock), kBlock, 0, st, d);
     return cudaGetLastError();
 }
 
 cudaError_t launch_merge_x(const Dev& d, double* x_aos, int first, int count, cudaStream_t st)
 {
-    if (count) k_merge_x<<<div_up(count, kBlock), kBlock, 0, st>>>(d, x_aos, first, count);
+    if (count) launch_dep(k_merge_x, div_up(count, kBlock), kBlock, 0, st, d, x_aos, first, count);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_partials(const Dev& d, int nblocks, int nvals, double* out, cudaStream_t st)
 {
-    k_reduce_partials<<<1, 1024, 0, st>>>(d.partial, nblocks, nvals, out);
+    launch_dep(k_reduce_partials, 1, 1024, 0, st, d.partial, nblocks, nvals, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_zero(double* a, size_t na, double* b, size_t nb, cudaStream_t st)
+{
+    if (na + nb) launch_dep(k_zero, div_up((long long)(na + nb), kBlock), kBlock, 0, st, a, na, b, nb);
     return cudaGetLastError();
 }
 

@@ -48,6 +48,7 @@
 
 #include "../../include/mapp_b200.h"
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 
 using namespace mg;
 
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(1024) k_lbfgs_step(Dev d, BatchView B, BatchPa
 // iteration budget lasts.
 __global__ void k_loop_test(BatchView B, cudaGraphConditionalHandle handle)
 {
+    dep_sync();
     __shared__ int sh_n;
     if (threadIdx.x == 0) sh_n = 0;
     __syncthreads();
@@ -500,13 +502,16 @@ __global__ void k_loop_test(BatchView B, cudaGraphConditionalHandle handle)
     }
 }
 
-__global__ void k_stamp(unsigned long long* t0) { *t0 = global_ns(); }
+__global__ void k_stamp(unsigned long long* t0) {
+    dep_sync(); *t0 = global_ns(); }
 
 // forces and densities of the running cells' sites to zero (a stopped cell
-// keeps the forces of its final point)
-__global__ void k_zero_active(Dev d)
+// keeps the forces of its final point), and every cell's energy
+__global__ void k_zero_active(Dev d, int ncells)
 {
+    dep_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ncells) d.cell_E[i] = 0.0;
     if (i >= d.natms || !d.cell_active[d.site_cell[i]]) return;
     for (int q = 0; q < d.x_dim; q++) d.f[(size_t)i * d.x_dim + q] = 0.0;
     for (int t = 0; t < d.nt; t++) d.E[(size_t)i * d.nt + t] = 0.0;
@@ -515,6 +520,7 @@ __global__ void k_zero_active(Dev d)
 // ghosts of running cells from their owners (position + image shift, alpha)
 __global__ void k_refresh_ghosts(Dev d, const double* __restrict__ shift, const unsigned char* __restrict__ active)
 {
+    dep_sync();
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= d.nph) return;
     const int g = d.natms + (int)k, o = d.root[g];
@@ -544,6 +550,7 @@ struct GatherDst {
 
 __global__ void k_gather_cell(Dev s, GatherDst D, int cell, int obase, int gbase, long long pbase)
 {
+    dep_sync();
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int nt = s.nt;
     if (k < s.nall) {
@@ -915,7 +922,7 @@ int build_all(mg_batch* b)
         D.natms_total = NT;
         const long long work = std::max<long long>((long long)d.nall, np);
         if (work > 0)
-            k_gather_cell<<<(unsigned)div_up(work, 256), 256, 0, bst>>>(d, D, c, b->h_base[c], ghost_fill, pair_fill);
+            launch_dep(k_gather_cell, (unsigned)div_up(work, 256), 256, 0, bst, d, D, c, b->h_base[c], ghost_fill, pair_fill);
         BCU(cudaGetLastError());
         ghost_fill += nph;
         pair_fill += np;
@@ -995,9 +1002,9 @@ int enqueue_iteration(mg_batch* b, cudaGraphConditionalHandle handle, bool with_
 {
     Dev& d = b->bd;
     cudaStream_t st = b->st;
-    if (d.nph > 0) k_refresh_ghosts<<<(unsigned)div_up(d.nph, 256), 256, 0, st>>>(d, b->shift.p, b->active.p);
-    if (d.natms > 0) k_zero_active<<<(unsigned)div_up(d.natms, 256), 256, 0, st>>>(d);
-    BCU(cudaMemsetAsync(d.cell_E, 0, b->cells.size() * sizeof(double), st));
+    if (d.nph > 0) launch_dep(k_refresh_ghosts, (unsigned)div_up(d.nph, 256), 256, 0, st, d, b->shift.p, b->active.p);
+    // (a cell has one site at least, so the sites' threads cover the cells)
+    launch_dep(k_zero_active, (unsigned)div_up(d.natms, 256), 256, 0, st, d, (int)b->cells.size());
     int rows = 0;
     if (d.npairs > 0) {
         if (b->form == MG_FORM_FP32) BCU(launch_dmd_force_f32(d, 0, &rows, st, nullptr));
@@ -1005,7 +1012,7 @@ int enqueue_iteration(mg_batch* b, cudaGraphConditionalHandle handle, bool with_
     }
     if (with_step) {
         BCU(launch_step(b->lcs, (int)b->cells.size(), b->lbt, st, d, view(b), params(b)));
-        k_loop_test<<<1, 256, 0, st>>>(view(b), handle);
+        launch_dep(k_loop_test, 1, 256, 0, st, view(b), handle);
         BCU(cudaGetLastError());
     }
     return MG_OK;
@@ -1415,7 +1422,7 @@ int mg_batch_relax(mg_batch* b, mg_batch_stats* stats)
     const int budget = (int)bud;
     int rounds = 0;
     auto t_start = std::chrono::steady_clock::now();
-    k_stamp<<<1, 1, 0, b->st>>>(b->t0.p);
+    launch_dep(k_stamp, 1, 1, 0, b->st, b->t0.p);
     std::vector<CellState> hs(ncells);
     for (;;) {
         BCU(cudaMemcpyAsync(b->budget.p, &budget, sizeof(int), cudaMemcpyHostToDevice, b->st));

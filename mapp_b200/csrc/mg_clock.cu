@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mg_internal.h"
+#include "mg_launch.cuh"
 #include "../../include/mapp_b200.h"
 
 namespace mg {
@@ -129,6 +130,7 @@ struct History {
 // a = -c - sum_j (delta_t beta[j+1]) y_j (clock_adams.cpp:205-213)
 __global__ void __launch_bounds__(kCkBlock) k_ck_form_a(CkView V, History Y)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     if (i >= V.n) return;
     double a = -V.c[i];
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kCkBlock) k_ck_form_a(CkView V, History Y)
 // the predictor's bound: min over i of the fraction of c_d dt that keeps c in [0, 1]
 __global__ void __launch_bounds__(kCkBlock) k_ck_predict_bound(CkView V, double dt)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[1] = {1.0};
     if (i < V.n) v[0] = box_bound(V.c[i], dadd(dmul(V.c_d[i], dt), V.c[i]), 1.0);
@@ -149,6 +152,7 @@ __global__ void __launch_bounds__(kCkBlock) k_ck_predict_bound(CkView V, double 
 // c += c_d dt ratio (clock_adams.cpp:277-283)
 __global__ void __launch_bounds__(kCkBlock) k_ck_predict(CkView V, double dt)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     if (i >= V.n) return;
     const double r = V.sc[SC_RATIO];
@@ -158,6 +162,7 @@ __global__ void __launch_bounds__(kCkBlock) k_ck_predict(CkView V, double dt)
 // g.g0 and g.g after the line search (clock_adams.cpp:340-352)
 __global__ void __launch_bounds__(kCkBlock) k_ck_dots(CkView V)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[2] = {0.0, 0.0};
     if (i < V.n) {
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(kCkBlock) k_ck_dots(CkView V)
 // clock_adams.cpp:287-314, clock_bdf.cpp:727-759
 __global__ void __launch_bounds__(kCkBlock) k_ck_first_dir(CkView V)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[2] = {0.0, 1.0};
     if (i < V.n) {
@@ -217,6 +223,7 @@ struct BdfHist {
 // y_0 and calc_g's a; SC_A receives -1 when some y_0 leaves [0, 1], else 1
 __global__ void __launch_bounds__(kCkBlock) k_bdf_interp(CkView V, BdfVecs B, BdfHist Y, double b_dady0, double ady0)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[1] = {1.0};
     if (i < V.n) {
@@ -239,6 +246,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bdf_interp(CkView V, BdfVecs B, Bd
 // 706-714)
 __global__ void __launch_bounds__(kCkBlock) k_bdf_predict_bound(CkView V, const double* y0, const double* dy, double dt)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[1] = {1.0};
     if (i < V.n) v[0] = box_bound(y0[i], dadd(dmul(dy[i], dt), y0[i]), 1.0);
@@ -249,6 +257,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bdf_predict_bound(CkView V, const 
 // c = y[0] + dy del_t ratio (clock_bdf.cpp:716-717)
 __global__ void __launch_bounds__(kCkBlock) k_bdf_predict(CkView V, const double* y0, const double* dy, double dt)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     if (i >= V.n) return;
     V.c[i] = dadd(y0[i], dmul(dmul(dy[i], dt), V.sc[SC_RATIO]));
@@ -258,6 +267,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bdf_predict(CkView V, const double
 // (clock_bdf.cpp:876-878): sum (y_0 - c)^2, sum c_d^2, count of c outside [0, 1]
 __global__ void __launch_bounds__(kCkBlock) k_bdf_err(CkView V, BdfVecs B)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[3] = {0.0, 0.0, 0.0};
     if (i < V.n) {
@@ -285,6 +295,7 @@ struct BdfHiLo {
 // higher- and lower-order error sums, then e_n = c - y_0
 __global__ void __launch_bounds__(kCkBlock) k_bdf_hilo(CkView V, BdfVecs B, BdfHiLo P)
 {
+    dep_sync();
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[2] = {0.0, 0.0};
     if (i < V.n) {
@@ -378,6 +389,7 @@ __device__ bool bs_outer_top(SolveDev& S)
 // after the first calc_g and the first direction (k_ck_first_dir)
 __global__ void k_bs_init(SolveDev* S, const double* red_out, const double* sc, cudaGraphConditionalHandle h)
 {
+    dep_sync();
     if (threadIdx.x) return;
     S->curr_cost = dmul(red_out[0], 0.25);
     S->g0_g0 = sc[SC_G0G0];
@@ -394,6 +406,7 @@ __global__ void k_bs_init(SolveDev* S, const double* red_out, const double* sc, 
 // search; ghosts from their owners (what the reference's refresh copies)
 __global__ void __launch_bounds__(kCkBlock) k_bs_trial(CkView V, const SolveDev* S)
 {
+    dep_sync();
     if (S->mode == 2) return;  // the full calc_g at the last point
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     const bool restore = S->mode == 1;
@@ -413,6 +426,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bs_trial(CkView V, const SolveDev*
 // (clock_bdf.cpp:760-806)
 __global__ void k_bs_post(SolveDev* S, const double* red_out, const double* sc)
 {
+    dep_sync();
     if (threadIdx.x) return;
     S->n_calc_g++;
     S->curr_cost = dmul(red_out[0], 0.25);
@@ -467,6 +481,7 @@ __global__ void k_bs_post(SolveDev* S, const double* red_out, const double* sc)
 // restarts from g when h.g < 0); only when the body's post step asked for it
 __global__ void __launch_bounds__(kCkBlock) k_bs_next_dir(CkView V, const SolveDev* S)
 {
+    dep_sync();
     if (!S->need_next) return;
     const double ratio = S->ratio;
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
@@ -493,6 +508,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bs_next_dir(CkView V, const SolveD
 // when h.g < 0 (clock_bdf.cpp:810-828), then the outer loop's test
 __global__ void k_bs_fin(SolveDev* S, const double* sc, cudaGraphConditionalHandle h)
 {
+    dep_sync();
     if (threadIdx.x) return;
     bool go = true;
     S->copy_hg = 0;
@@ -518,6 +534,7 @@ __global__ void k_bs_fin(SolveDev* S, const double* sc, cudaGraphConditionalHand
 
 __global__ void __launch_bounds__(kCkBlock) k_bs_copy(CkView V, const SolveDev* S)
 {
+    dep_sync();
     if (!S->copy_hg) return;
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     if (i < V.n) V.h[i] = V.g[i];
@@ -586,15 +603,15 @@ struct Clock {
     // update, the outer loop's test
     int enqueue_ls_body(cudaGraphConditionalHandle h)
     {
-        k_bs_trial<<<trial_grid(), kCkBlock, 0, st>>>(V, S_dev);
+        launch_dep(k_bs_trial, trial_grid(), kCkBlock, 0, st, V, S_dev);
         KCU(cudaGetLastError());
         int rows = 0;
         KCHK(system_enqueue_calc_g_dev(s, &S_dev->calc_chk, &S_dev->alpha, &rows));
-        k_ck_dots<<<grid(), kCkBlock, 0, st>>>(V);
-        k_bs_post<<<1, 32, 0, st>>>(S_dev, system_red_out(s), V.sc);
-        k_bs_next_dir<<<grid(), kCkBlock, 0, st>>>(V, S_dev);
-        k_bs_fin<<<1, 32, 0, st>>>(S_dev, V.sc, h);
-        k_bs_copy<<<grid(), kCkBlock, 0, st>>>(V, S_dev);
+        launch_dep(k_ck_dots, grid(), kCkBlock, 0, st, V);
+        launch_dep(k_bs_post, 1, 32, 0, st, S_dev, system_red_out(s), V.sc);
+        launch_dep(k_bs_next_dir, grid(), kCkBlock, 0, st, V, S_dev);
+        launch_dep(k_bs_fin, 1, 32, 0, st, S_dev, V.sc, h);
+        launch_dep(k_bs_copy, grid(), kCkBlock, 0, st, V, S_dev);
         KCU(cudaGetLastError());
         return MG_OK;
     }
@@ -662,12 +679,12 @@ struct Clock {
         KCHK(system_enqueue_calc_g(s, 0, alpha, &rows));
         n_calc_g++;
         KCHK(system_enqueue_c_d(s));
-        k_ck_predict_bound<<<grid(), kCkBlock, 0, st>>>(V, delta_t);
-        k_ck_predict<<<grid(), kCkBlock, 0, st>>>(V, delta_t);
+        launch_dep(k_ck_predict_bound, grid(), kCkBlock, 0, st, V, delta_t);
+        launch_dep(k_ck_predict, grid(), kCkBlock, 0, st, V, delta_t);
         KCU(cudaGetLastError());
         KCHK(refresh_c());
         // h = g, and the first iteration's g0, c0 and step bound with it
-        k_ck_first_dir<<<grid(), kCkBlock, 0, st>>>(V);
+        launch_dep(k_ck_first_dir, grid(), kCkBlock, 0, st, V);
         KCU(cudaGetLastError());
         SolveDev hs{};
         hs.tol = 1.0e-8;
@@ -736,7 +753,7 @@ struct Bdf {
             H.ay[j] = alpha_y[j];
             H.bdy[j] = beta * dalpha_y[j];
         }
-        k_bdf_interp<<<grid(), kCkBlock, 0, ck->st>>>(ck->V, B, H, beta * dalpha_dy_0, alpha_dy_0);
+        launch_dep(k_bdf_interp, grid(), kCkBlock, 0, ck->st, ck->V, B, H, beta * dalpha_dy_0, alpha_dy_0);
         KCU(cudaGetLastError());
         KCHK(ck->read_scalars());
         *ret = ck->host_sc[SC_A] < 0.0 ? -1 : 1;
@@ -752,15 +769,15 @@ struct Bdf {
     int solve(double del_t, int q, double* out)
     {
         const mg_bdf_opts& o = p;
-        k_bdf_predict_bound<<<grid(), kCkBlock, 0, ck->st>>>(ck->V, y[0], B.dy, del_t);
-        k_bdf_predict<<<grid(), kCkBlock, 0, ck->st>>>(ck->V, y[0], B.dy, del_t);
+        launch_dep(k_bdf_predict_bound, grid(), kCkBlock, 0, ck->st, ck->V, y[0], B.dy, del_t);
+        launch_dep(k_bdf_predict, grid(), kCkBlock, 0, ck->st, ck->V, y[0], B.dy, del_t);
         KCU(cudaGetLastError());
         KCHK(ck->refresh_c());
         int rows = 0;
         KCHK(system_enqueue_calc_g(ck->s, 0, beta, &rows));
         ck->n_calc_g++;
         // h = g, and the first iteration's g0, c0 and step bound with it
-        k_ck_first_dir<<<grid(), kCkBlock, 0, ck->st>>>(ck->V);
+        launch_dep(k_ck_first_dir, grid(), kCkBlock, 0, ck->st, ck->V);
         KCU(cudaGetLastError());
         SolveDev hs{};
         hs.tol = o.m_tol * (double)dof_tot;
@@ -771,7 +788,7 @@ struct Bdf {
         hs.max_iter = o.max_iter;
         KCU(cudaMemcpyAsync(ck->S_dev, &hs, sizeof(SolveDev), cudaMemcpyHostToDevice, ck->st));
         KCU(cudaGraphLaunch(ck->ls_exec, ck->st));
-        k_bdf_err<<<grid(), kCkBlock, 0, ck->st>>>(ck->V, B);
+        launch_dep(k_bdf_err, grid(), kCkBlock, 0, ck->st, ck->V, B);
         KCU(cudaGetLastError());
         // the line search's state and the error sums in one synchronisation
         KCU(cudaMemcpyAsync(&ck->hout->r, ck->S_dev, sizeof(SolveDev), cudaMemcpyDeviceToHost, ck->st));
@@ -842,7 +859,7 @@ struct Bdf {
         }
         P.hi = hi_ord_avail;
         P.lo = lo_ord_avail;
-        k_bdf_hilo<<<grid(), kCkBlock, 0, ck->st>>>(ck->V, B, P);
+        launch_dep(k_bdf_hilo, grid(), kCkBlock, 0, ck->st, ck->V, B, P);
         KCU(cudaGetLastError());
         // the error sums only steer an order change: with neither order
         // available the host has nothing to read (the kernel still updates
@@ -985,7 +1002,7 @@ extern "C" int mg_clock_adams(mg_system* s, int order, int nsteps, double delta_
             }
             bet = beta[0];
         }
-        k_ck_form_a<<<nblocks, kCkBlock, 0, ck.st>>>(ck.V, Y);
+        launch_dep(k_ck_form_a, nblocks, kCkBlock, 0, ck.st, ck.V, Y);
         KCU(cudaGetLastError());
         double cur = 0.0;
         KCHK(ck.solve(delta_t, bet, &cur));
@@ -1080,7 +1097,7 @@ extern "C" int mg_clock_bdf(mg_system* s, int nsteps, const mg_bdf_opts* opts, d
     double initial_del_t = o.initial_del_t;
     if (initial_del_t < 0.0) {
         // y_0 is still zero: the error kernel's second sum is sum c_d^2
-        k_bdf_err<<<nblocks, kCkBlock, 0, ck.st>>>(ck.V, b.B);
+        launch_dep(k_bdf_err, nblocks, kCkBlock, 0, ck.st, ck.V, b.B);
         KCU(cudaGetLastError());
         KCHK(ck.read_scalars());
         double sum = sqrt(ck.host_sc[SC_GG] / (double)n);

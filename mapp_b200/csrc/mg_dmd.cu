@@ -16,6 +16,7 @@
 // alpha outside (alpha_min, alpha_max), no node inside the table) are written
 // as zero, so results never depend on earlier calls.
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 #include "mg_dmd_common.cuh"
 
 namespace mg {
@@ -37,6 +38,7 @@ namespace {
 template <int NT, int NQ>
 __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_pass1(Dev d, int row0)
 {
+    dep_sync();
     using S = Slots<NT>;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_pass1(Dev d, int 
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_dmd_embed(Dev d, int with_force, int row0)
 {
+    dep_sync();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = idx / NT, a = idx - (idx / NT) * NT;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -155,6 +158,7 @@ __global__ void __launch_bounds__(kFFBlock) k_dmd_embed(Dev d, int with_force, i
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_pass2(Dev d, int st_clc, int row0)
 {
+    dep_sync();
     using S = Slots<NT>;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -263,6 +267,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_pass2(Dev d, int 
 template <int NT, int NQ>
 __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_energy_pass(Dev d, int row0)
 {
+    dep_sync();
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -328,6 +333,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_DMD_MINB) k_dmd_energy_pass(Dev d
 // ---- create_2nd_neigh_lst (ff_dmd_I.cpp:2138-2217) ------------------------
 __global__ void __launch_bounds__(kFFBlock) k_dmd_crd(Dev d)
 {
+    dep_sync();
     int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (i >= d.natms) return;
@@ -366,6 +372,7 @@ __global__ void __launch_bounds__(kFFBlock) k_dmd_crd(Dev d)
 
 __global__ void k_crd_ghosts(Dev d)
 {
+    dep_sync();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < d.nph) d.crd[d.natms + k] = d.crd[d.root[d.natms + k]];
 }
@@ -387,6 +394,7 @@ constexpr int kCrdLanes = MG_CRD_LANES;
 template <int NT, typename P, int G>
 __global__ void __launch_bounds__(kFFBlock) k_mu_E(Dev d)
 {
+    dep_sync();
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     int lane = threadIdx.x & (G - 1);
     if (i >= d.natms) return;
@@ -431,6 +439,7 @@ __global__ void __launch_bounds__(kFFBlock) k_mu_E(Dev d)
 template <int NT>
 __global__ void k_mu_embed(Dev d, int with_dd)
 {
+    dep_sync();
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= d.natms * NT) return;
     int a = idx % NT;
@@ -455,6 +464,7 @@ __device__ __forceinline__ double dE_flat(const Dev& d, int q)
 template <int NT, typename P, int G>
 __global__ void __launch_bounds__(kFFBlock) k_mu_npairs(Dev d)
 {
+    dep_sync();
     using S = Slots<NT>;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     int lane = threadIdx.x & (G - 1);
@@ -526,6 +536,7 @@ __device__ __forceinline__ void mu_nfinal(const Dev& d, int idx, int mode)
 template <int NT>
 __global__ void k_mu_nfinal(Dev d, int mode)
 {
+    dep_sync();
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < d.natms * NT) mu_nfinal<NT>(d, idx, mode);
 }
@@ -556,6 +567,7 @@ __device__ __forceinline__ double rate_sij(const Dev& d, double ni, double nj, d
 template <int NT, int G>
 __global__ void __launch_bounds__(kFFBlock) k_cd_rates(Dev d)
 {
+    dep_sync();
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     int lane = threadIdx.x & (G - 1);
     if (i >= d.natms) return;
@@ -590,6 +602,7 @@ __global__ void __launch_bounds__(kFFBlock) k_cd_rates(Dev d)
 template <int NT>
 __global__ void k_g_sinit(Dev d, int mode)
 {
+    dep_sync();
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= d.natms * NT) return;
     mu_nfinal<NT>(d, idx, mode);
@@ -600,6 +613,7 @@ __global__ void k_g_sinit(Dev d, int mode)
 template <int NT, int G>
 __global__ void __launch_bounds__(kFFBlock) k_g_srates(Dev d, double alpha)
 {
+    dep_sync();
     if (d.g_alpha) alpha = *d.g_alpha;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     int lane = threadIdx.x & (G - 1);
@@ -643,6 +657,7 @@ __global__ void __launch_bounds__(kFFBlock) k_g_srates(Dev d, double alpha)
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_g_cost(Dev d, int row0, int chk)
 {
+    dep_sync();
     if (d.g_chk) chk = *d.g_chk;
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -663,6 +678,7 @@ __global__ void __launch_bounds__(kFFBlock) k_g_cost(Dev d, int row0, int chk)
 template <int NT, int G>
 __global__ void __launch_bounds__(kFFBlock) k_g_trates(Dev d, double alpha)
 {
+    dep_sync();
     if (d.g_chk && *d.g_chk) return;  // cost-only call: no g terms
     if (d.g_alpha) alpha = *d.g_alpha;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -733,6 +749,7 @@ __global__ void __launch_bounds__(kFFBlock) k_g_trates(Dev d, double alpha)
 template <int NT, typename P, int G>
 __global__ void __launch_bounds__(kFFBlock) k_g_vpass(Dev d, double alpha)
 {
+    dep_sync();
     if (d.g_chk && *d.g_chk) return;  // cost-only call: no g terms
     if (d.g_alpha) alpha = *d.g_alpha;
     using S = Slots<NT>;
@@ -795,6 +812,7 @@ __global__ void __launch_bounds__(kFFBlock) k_g_vpass(Dev d, double alpha)
 template <int NT, typename P, int G>
 __global__ void __launch_bounds__(kFFBlock) k_g_last(Dev d, double alpha)
 {
+    dep_sync();
     if (d.g_chk && *d.g_chk) return;  // cost-only call: no g terms
     if (d.g_alpha) alpha = *d.g_alpha;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -862,6 +880,7 @@ __device__ __forceinline__ bool pair_active(const Dev& d, long long slot)
 template <int NT>
 __global__ void k_active_count(Dev d)
 {
+    dep_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) d.nact[d.natms] = 0;
     if (i >= d.natms) return;
@@ -874,6 +893,7 @@ __global__ void k_active_count(Dev d)
 template <int NT>
 __global__ void k_active_fill(Dev d)
 {
+    dep_sync();
     using S = Slots<NT>;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.natms) return;
@@ -898,12 +918,12 @@ cudaError_t dmd_force_nt(const Dev& d, int st_clc, int* nb, cudaStream_t st, cud
     int g1 = persistent_grid(d.npairs, d.tune_bps > 0 ? d.tune_bps : MG_DMD_MINB), g2 = div_up(d.natms * NT, kFFBlock);
     int g3 = persistent_grid(d.npairs, d.tune_bps2 > 0 ? d.tune_bps2 : MG_DMD_MINB);
     if (evs) cudaEventRecord(evs[0], st);
-    if (d.nq == 3) k_dmd_pass1<NT, 3><<<g1, kFFBlock, 0, st>>>(d, 0);
-    else k_dmd_pass1<NT, 0><<<g1, kFFBlock, 0, st>>>(d, 0);
+    if (d.nq == 3) launch_dep(k_dmd_pass1<NT, 3>, g1, kFFBlock, 0, st, d, 0);
+    else launch_dep(k_dmd_pass1<NT, 0>, g1, kFFBlock, 0, st, d, 0);
     if (evs) cudaEventRecord(evs[1], st);
-    k_dmd_embed<NT><<<g2, kFFBlock, 0, st>>>(d, 1, g1);
+    launch_dep(k_dmd_embed<NT>, g2, kFFBlock, 0, st, d, 1, g1);
     if (evs) cudaEventRecord(evs[2], st);
-    k_dmd_pass2<NT><<<g3, kFFBlock, 0, st>>>(d, st_clc, g1 + g2);
+    launch_dep(k_dmd_pass2<NT>, g3, kFFBlock, 0, st, d, st_clc, g1 + g2);
     if (evs) cudaEventRecord(evs[3], st);
     *nb = g1 + g2 + g3;
     return cudaGetLastError();
@@ -913,9 +933,9 @@ template <int NT>
 cudaError_t dmd_energy_nt(const Dev& d, int* nb, cudaStream_t st)
 {
     int g1 = persistent_grid(d.npairs, MG_DMD_MINB), g2 = div_up(d.natms * NT, kFFBlock);
-    if (d.nq == 3) k_dmd_energy_pass<NT, 3><<<g1, kFFBlock, 0, st>>>(d, 0);
-    else k_dmd_energy_pass<NT, 0><<<g1, kFFBlock, 0, st>>>(d, 0);
-    k_dmd_embed<NT><<<g2, kFFBlock, 0, st>>>(d, 0, g1);
+    if (d.nq == 3) launch_dep(k_dmd_energy_pass<NT, 3>, g1, kFFBlock, 0, st, d, 0);
+    else launch_dep(k_dmd_energy_pass<NT, 0>, g1, kFFBlock, 0, st, d, 0);
+    launch_dep(k_dmd_embed<NT>, g2, kFFBlock, 0, st, d, 0, g1);
     *nb = g1 + g2;
     return cudaGetLastError();
 }
@@ -925,11 +945,11 @@ cudaError_t dmd_cdot_ntp(const Dev& d, cudaStream_t st)
 {
     int gw = div_up((long long)d.natms * kNbrLanes, kFFBlock), gc = div_up((long long)d.natms * kCrdLanes, kFFBlock);
     int gs = div_up((long long)d.natms * NT, kFFBlock);
-    k_mu_E<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d);
-    k_mu_embed<NT><<<gs, kFFBlock, 0, st>>>(d, 0);
-    k_mu_npairs<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d);
-    k_mu_nfinal<NT><<<gs, kFFBlock, 0, st>>>(d, d.style == STYLE_DMD_II ? 1 : 0);
-    k_cd_rates<NT, kCrdLanes><<<gc, kFFBlock, 0, st>>>(d);
+    launch_dep(k_mu_E<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d);
+    launch_dep(k_mu_embed<NT>, gs, kFFBlock, 0, st, d, 0);
+    launch_dep(k_mu_npairs<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d);
+    launch_dep(k_mu_nfinal<NT>, gs, kFFBlock, 0, st, d, d.style == STYLE_DMD_II ? 1 : 0);
+    launch_dep(k_cd_rates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d);
     return cudaGetLastError();
 }
 
@@ -944,17 +964,17 @@ cudaError_t dmd_calc_g_ntp(const Dev& d, int chk, double alpha, int* nb, cudaStr
 {
     int gw = div_up((long long)d.natms * kNbrLanes, kFFBlock), gc = div_up((long long)d.natms * kCrdLanes, kFFBlock);
     int gs = div_up((long long)d.natms * NT, kFFBlock);
-    k_mu_E<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d);
-    k_mu_embed<NT><<<gs, kFFBlock, 0, st>>>(d, 1);
-    k_mu_npairs<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d);
-    k_g_sinit<NT><<<gs, kFFBlock, 0, st>>>(d, d.style == STYLE_DMD_II ? 3 : 2);
-    k_g_srates<NT, kCrdLanes><<<gc, kFFBlock, 0, st>>>(d, alpha);
-    k_g_cost<NT><<<gs, kFFBlock, 0, st>>>(d, 0, chk);
+    launch_dep(k_mu_E<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d);
+    launch_dep(k_mu_embed<NT>, gs, kFFBlock, 0, st, d, 1);
+    launch_dep(k_mu_npairs<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d);
+    launch_dep(k_g_sinit<NT>, gs, kFFBlock, 0, st, d, d.style == STYLE_DMD_II ? 3 : 2);
+    launch_dep(k_g_srates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d, alpha);
+    launch_dep(k_g_cost<NT>, gs, kFFBlock, 0, st, d, 0, chk);
     *nb = gs;
     if (!chk || d.g_chk) {
-        k_g_trates<NT, kCrdLanes><<<gc, kFFBlock, 0, st>>>(d, alpha);
-        k_g_vpass<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d, alpha);
-        k_g_last<NT, P, kNbrLanes><<<gw, kFFBlock, 0, st>>>(d, alpha);
+        launch_dep(k_g_trates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d, alpha);
+        launch_dep(k_g_vpass<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d, alpha);
+        launch_dep(k_g_last<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d, alpha);
     }
     return cudaGetLastError();
 }
@@ -992,8 +1012,8 @@ cudaError_t launch_dmd_energy(const Dev& d, int* nb, cudaStream_t st)
 
 cudaError_t launch_dmd_crd(const Dev& d, cudaStream_t st)
 {
-    if (d.natms) k_dmd_crd<<<div_up((long long)d.natms * 32, kFFBlock), kFFBlock, 0, st>>>(d);
-    if (d.nph) k_crd_ghosts<<<div_up(d.nph, kFFBlock), kFFBlock, 0, st>>>(d);
+    if (d.natms) launch_dep(k_dmd_crd, div_up((long long)d.natms * 32, kFFBlock), kFFBlock, 0, st, d);
+    if (d.nph) launch_dep(k_crd_ghosts, div_up(d.nph, kFFBlock), kFFBlock, 0, st, d);
     return cudaGetLastError();
 }
 
@@ -1012,10 +1032,10 @@ cudaError_t launch_active_count(const Dev& d, cudaStream_t st)
 {
     const int g = div_up(d.natms + 1, kFFBlock);
     switch (d.nt) {
-    case 1: k_active_count<1><<<g, kFFBlock, 0, st>>>(d); break;
-    case 2: k_active_count<2><<<g, kFFBlock, 0, st>>>(d); break;
-    case 3: k_active_count<3><<<g, kFFBlock, 0, st>>>(d); break;
-    case 4: k_active_count<4><<<g, kFFBlock, 0, st>>>(d); break;
+    case 1: launch_dep(k_active_count<1>, g, kFFBlock, 0, st, d); break;
+    case 2: launch_dep(k_active_count<2>, g, kFFBlock, 0, st, d); break;
+    case 3: launch_dep(k_active_count<3>, g, kFFBlock, 0, st, d); break;
+    case 4: launch_dep(k_active_count<4>, g, kFFBlock, 0, st, d); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -1025,10 +1045,10 @@ cudaError_t launch_active_fill(const Dev& d, cudaStream_t st)
 {
     const int g = div_up(d.natms, kFFBlock);
     switch (d.nt) {
-    case 1: k_active_fill<1><<<g, kFFBlock, 0, st>>>(d); break;
-    case 2: k_active_fill<2><<<g, kFFBlock, 0, st>>>(d); break;
-    case 3: k_active_fill<3><<<g, kFFBlock, 0, st>>>(d); break;
-    case 4: k_active_fill<4><<<g, kFFBlock, 0, st>>>(d); break;
+    case 1: launch_dep(k_active_fill<1>, g, kFFBlock, 0, st, d); break;
+    case 2: launch_dep(k_active_fill<2>, g, kFFBlock, 0, st, d); break;
+    case 3: launch_dep(k_active_fill<3>, g, kFFBlock, 0, st, d); break;
+    case 4: launch_dep(k_active_fill<4>, g, kFFBlock, 0, st, d); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -48,6 +48,7 @@
 #include <unordered_map>
 
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 #include "mg_dmd_common.cuh"
 #include "mg_split.cuh"
 
@@ -153,6 +154,7 @@ __device__ __forceinline__ void load_rec(const Dev& d, int j, float (&al)[NT], f
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_dmd32_prep(Dev d)
 {
+    dep_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) d.status[4] = 0;
     if (i < d.nall) {
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(kFFBlock) k_dmd32_prep(Dev d)
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_dmd32_fmerge(Dev d)
 {
+    dep_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.natms || !site_active(d, i)) return;
     const float4 a = reinterpret_cast<const float4*>(d.facc)[(size_t)i * 2];
@@ -194,6 +197,7 @@ constexpr int kQueue = 64;  // per-warp queue of in-cut pairs (two batches)
 template <int NT, int NQ>
 __global__ void MG_DENS_BOUNDS k_dmd32_dens(Dev d, int K)
 {
+    dep_sync();
     extern __shared__ float4 tab[];
     __shared__ int2 q_ij[kFFWarps][kQueue];
     __shared__ float4 q_x[kFFWarps][kQueue];  // dx, dy, dz (FP32), rsq
@@ -347,6 +351,7 @@ __global__ void MG_DENS_BOUNDS k_dmd32_dens(Dev d, int K)
 template <int NT, int NQ>
 __global__ void MG_FORCE_BOUNDS k_dmd32_force(Dev d, int st_clc, int row0, int W, int K)
 {
+    dep_sync();
     using S = Slots<NT>;
     extern __shared__ float4 tab[];
     load_split_table(d, tab, NT * NT + S::NC);
@@ -511,6 +516,7 @@ __global__ void MG_FORCE_BOUNDS k_dmd32_force(Dev d, int st_clc, int row0, int W
 template <int NT, int NQ>
 __global__ void __launch_bounds__(kFFBlock) k_dmd32_fill(Dev d)
 {
+    dep_sync();
     using S = Slots<NT>;
     extern __shared__ float4 tab[];
     load_split_table(d, tab, NT * NT + S::NC);
@@ -559,6 +565,7 @@ __global__ void __launch_bounds__(kFFBlock) k_dmd32_fill(Dev d)
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_dmd32_embed(Dev d, int row0)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     double e = 0.0;
@@ -588,6 +595,7 @@ __global__ void __launch_bounds__(kFFBlock) k_dmd32_embed(Dev d, int row0)
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock, MG_DMD32_MINB) k_dmd32_pass2(Dev d, int st_clc, int row0)
 {
+    dep_sync();
     using S = Slots<NT>;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -742,13 +750,13 @@ cudaError_t dmd32_force_nt(const Dev& d, int st_clc, int* nb, cudaStream_t st, c
     const int W = gA * kFFWarps;
     const int K = (int)std::max(1LL, (d.npairs + (long long)gA * kFFBlock - 1) / ((long long)gA * kFFBlock));
     if ((long long)W * K * 32 > d.icut_cap || W > dmd32_icut_warps()) return cudaErrorInvalidValue;
-    k_dmd32_prep<NT><<<g0, kFFBlock, 0, st>>>(d);
-    kA<<<gA, kFFBlock, smA, st>>>(d, K);
+    launch_dep(k_dmd32_prep<NT>, g0, kFFBlock, 0, st, d);
+    launch_full(kA, gA, kFFBlock, smA, st, d, K);
     if (evs) cudaEventRecord(evs[1], st);
-    k_dmd32_embed<NT><<<g2, kFFBlock, 0, st>>>(d, 0);
+    launch_dep(k_dmd32_embed<NT>, g2, kFFBlock, 0, st, d, 0);
     if (evs) cudaEventRecord(evs[2], st);
-    kB<<<gB, kFFBlock, smB, st>>>(d, st_clc, g2, W, K);
-    k_dmd32_fmerge<NT><<<g2, kFFBlock, 0, st>>>(d);
+    launch_full(kB, gB, kFFBlock, smB, st, d, st_clc, g2, W, K);
+    launch_dep(k_dmd32_fmerge<NT>, g2, kFFBlock, 0, st, d);
     if (evs) cudaEventRecord(evs[3], st);
     *nb = g2 + gB;
     return cudaGetLastError();
@@ -765,7 +773,7 @@ cudaError_t dmd32_fill_nt(const Dev& d, cudaStream_t st)
     void (*kf)(Dev) = mid0 ? k_dmd32_fill<NT, 3> : k_dmd32_fill<NT, 0>;
     const int r = resident_blocks((const void*)kf, sm);
     if (r == 0) return cudaErrorInvalidConfiguration;
-    kf<<<pair_grid(d.npairs, r, 0), kFFBlock, sm, st>>>(d);
+    launch_full(kf, pair_grid(d.npairs, r, 0), kFFBlock, sm, st, d);
     return cudaGetLastError();
 }
 
@@ -773,9 +781,9 @@ template <int NT>
 cudaError_t dmd32_tail_nt(const Dev& d, int st_clc, int row0, int* nb, cudaStream_t st, cudaEvent_t* evs)
 {
     int g1 = persistent_grid(d.npairs, d.tune_bps2 > 0 ? d.tune_bps2 : MG_DMD32_MINB), g2 = div_up(d.natms, kFFBlock);
-    k_dmd32_embed<NT><<<g2, kFFBlock, 0, st>>>(d, row0);
+    launch_dep(k_dmd32_embed<NT>, g2, kFFBlock, 0, st, d, row0);
     if (evs) cudaEventRecord(evs[2], st);
-    k_dmd32_pass2<NT><<<g1, kFFBlock, 0, st>>>(d, st_clc, row0 + g2);
+    launch_dep(k_dmd32_pass2<NT>, g1, kFFBlock, 0, st, d, st_clc, row0 + g2);
     if (evs) cudaEventRecord(evs[3], st);
     *nb = g1 + g2;
     return cudaGetLastError();

@@ -23,6 +23,7 @@
 // coefficients, one species needs no gather, and the reductions share lines:
 // 177 us and 115 us (L1 data stage 84 % and 76 % busy; 798 -> 352 us a call).
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 #include "mg_dmd_common.cuh"
 
 namespace mg {
@@ -69,6 +70,7 @@ __device__ __forceinline__ void add_virial(double (&acc)[7], double w, double dx
 template <bool kEnergyOnly, bool kOne>
 __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_eam_pass1(Dev d, int st_clc, int row0)
 {
+    dep_sync();
     constexpr int NV = kEnergyOnly ? 1 : 4;
     __shared__ RowBuf<NV> sh[kFFWarps];
     RowBuf<NV>& buf = sh[threadIdx.x >> 5];
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_eam_pass1(Dev d, int 
 template <bool kEnergyOnly>
 __global__ void __launch_bounds__(kFFBlock) k_eam_embed(Dev d, int row0)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (i < d.natms) {
@@ -158,6 +161,7 @@ __global__ void __launch_bounds__(kFFBlock) k_eam_embed(Dev d, int row0)
 // (ff_eam.cpp:196-250, ff_fs.cpp:531-588).
 __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_embed_pass2(Dev d, int st_clc, int row0)
 {
+    dep_sync();
     constexpr int NV = 3;
     __shared__ RowBuf<NV> sh[kFFWarps];
     RowBuf<NV>& buf = sh[threadIdx.x >> 5];
@@ -191,6 +195,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_embed_pass2(Dev d, in
 template <bool kEnergyOnly>
 __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_fs_pass1(Dev d, int st_clc, int row0)
 {
+    dep_sync();
     constexpr int NV = kEnergyOnly ? 1 : 4;
     __shared__ RowBuf<NV> sh[kFFWarps];
     RowBuf<NV>& buf = sh[threadIdx.x >> 5];
@@ -254,6 +259,7 @@ __global__ void __launch_bounds__(kFFBlock, MG_EAM_MINB) k_fs_pass1(Dev d, int s
 template <bool kEnergyOnly>
 __global__ void __launch_bounds__(kFFBlock) k_fs_embed(Dev d, int row0)
 {
+    dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (i < d.natms) {
@@ -270,10 +276,10 @@ __global__ void __launch_bounds__(kFFBlock) k_fs_embed(Dev d, int row0)
 cudaError_t launch_eam_force(const Dev& d, int st_clc, int* nblocks_out, cudaStream_t st)
 {
     const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
-    if (d.nt == 1) k_eam_pass1<false, true><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
-    else k_eam_pass1<false, false><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
-    k_eam_embed<false><<<g2, kFFBlock, 0, st>>>(d, g1);
-    k_embed_pass2<<<g1, kFFBlock, 0, st>>>(d, st_clc, g1 + g2);
+    if (d.nt == 1) launch_dep(k_eam_pass1<false, true>, g1, kFFBlock, 0, st, d, st_clc, 0);
+    else launch_dep(k_eam_pass1<false, false>, g1, kFFBlock, 0, st, d, st_clc, 0);
+    launch_dep(k_eam_embed<false>, g2, kFFBlock, 0, st, d, g1);
+    launch_dep(k_embed_pass2, g1, kFFBlock, 0, st, d, st_clc, g1 + g2);
     *nblocks_out = 2 * g1 + g2;
     return cudaGetLastError();
 }
@@ -281,9 +287,9 @@ cudaError_t launch_eam_force(const Dev& d, int st_clc, int* nblocks_out, cudaStr
 cudaError_t launch_eam_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 {
     const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
-    if (d.nt == 1) k_eam_pass1<true, true><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
-    else k_eam_pass1<true, false><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
-    k_eam_embed<true><<<g2, kFFBlock, 0, st>>>(d, g1);
+    if (d.nt == 1) launch_dep(k_eam_pass1<true, true>, g1, kFFBlock, 0, st, d, 0, 0);
+    else launch_dep(k_eam_pass1<true, false>, g1, kFFBlock, 0, st, d, 0, 0);
+    launch_dep(k_eam_embed<true>, g2, kFFBlock, 0, st, d, g1);
     *nblocks_out = g1 + g2;
     return cudaGetLastError();
 }
@@ -291,9 +297,9 @@ cudaError_t launch_eam_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 cudaError_t launch_fs_force(const Dev& d, int st_clc, int* nblocks_out, cudaStream_t st)
 {
     const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
-    k_fs_pass1<false><<<g1, kFFBlock, 0, st>>>(d, st_clc, 0);
-    k_fs_embed<false><<<g2, kFFBlock, 0, st>>>(d, g1);
-    k_embed_pass2<<<g1, kFFBlock, 0, st>>>(d, st_clc, g1 + g2);
+    launch_dep(k_fs_pass1<false>, g1, kFFBlock, 0, st, d, st_clc, 0);
+    launch_dep(k_fs_embed<false>, g2, kFFBlock, 0, st, d, g1);
+    launch_dep(k_embed_pass2, g1, kFFBlock, 0, st, d, st_clc, g1 + g2);
     *nblocks_out = 2 * g1 + g2;
     return cudaGetLastError();
 }
@@ -301,8 +307,8 @@ cudaError_t launch_fs_force(const Dev& d, int st_clc, int* nblocks_out, cudaStre
 cudaError_t launch_fs_energy(const Dev& d, int* nblocks_out, cudaStream_t st)
 {
     const int g1 = persistent_grid(d.npairs, MG_EAM_MINB), g2 = div_up(d.natms, kFFBlock);
-    k_fs_pass1<true><<<g1, kFFBlock, 0, st>>>(d, 0, 0);
-    k_fs_embed<true><<<g2, kFFBlock, 0, st>>>(d, g1);
+    launch_dep(k_fs_pass1<true>, g1, kFFBlock, 0, st, d, 0, 0);
+    launch_dep(k_fs_embed<true>, g2, kFFBlock, 0, st, d, g1);
     *nblocks_out = g1 + g2;
     return cudaGetLastError();
 }

@@ -256,6 +256,8 @@ cudaError_t launch_update_x(const Dev& d, const double* x_aos, double sq_skin, i
 cudaError_t launch_refresh_c(const Dev& d, cudaStream_t st);
 cudaError_t launch_merge_x(const Dev& d, double* x_aos, int first, int count, cudaStream_t st);
 cudaError_t launch_reduce_partials(const Dev& d, int nblocks, int nvals, double* out, cudaStream_t st);
+// zeroes a[0..na) and b[0..nb)
+cudaError_t launch_zero(double* a, size_t na, double* b, size_t nb, cudaStream_t st);
 size_t scan_temp_bytes(int n);
 cudaError_t launch_exclusive_scan(const int* in, int* out, int n, void* temp, size_t temp_bytes, cudaStream_t st);
 // EAM / FS

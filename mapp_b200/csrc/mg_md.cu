@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "mg_internal.h"
+#include "mg_launch.cuh"
 #include "../../include/mapp_b200.h"
 
 namespace mg {
@@ -157,6 +158,7 @@ __device__ bool last_block_sum(double (&v)[NV], double* __restrict__ part, unsig
 // start of the very first step: the thermostat's first half step
 __global__ void k_md_begin(NhState* S, NhConst C)
 {
+    dep_sync();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         S->fac_a = 1.0;
         S->fac_b = nh_chain(S, C, C.dt2);
@@ -168,6 +170,7 @@ __global__ void k_md_begin(NhState* S, NhConst C)
 __global__ void __launch_bounds__(kMdBlock) k_md_kick_drift(Dev d, NhConst C, NhState* S, double4* __restrict__ xd,
                                                             double4* __restrict__ xu, double* __restrict__ part)
 {
+    dep_sync();
     if (S->done) return;
     const int i = blockIdx.x * kMdBlock + threadIdx.x;
     const double fa = S->fac_a, fb = S->fac_b;
@@ -202,6 +205,7 @@ __global__ void __launch_bounds__(kMdBlock) k_md_center(Dev d, NhConst C, NhStat
                                                         const double4* __restrict__ xu,
                                                         cudaGraphConditionalHandle handle, int set_cond)
 {
+    dep_sync();
     __shared__ bool last;
     if (S->done) {
         if (set_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(kMdBlock) k_md_center(Dev d, NhConst C, NhStat
 __global__ void __launch_bounds__(kMdBlock) k_md_kick2(Dev d, NhConst C, NhState* S, double4* __restrict__ xd,
                                                        double* __restrict__ part)
 {
+    dep_sync();
     const int i = blockIdx.x * kMdBlock + threadIdx.x;
     double t[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (i < d.natms) {
@@ -282,6 +287,7 @@ __global__ void __launch_bounds__(kMdBlock) k_md_kick2(Dev d, NhConst C, NhState
 // the last step's pending rescale
 __global__ void k_md_finish(Dev d, NhState* S, double4* __restrict__ xd)
 {
+    dep_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.natms) return;
     const double fa = S->fac_a;
@@ -363,9 +369,9 @@ int enqueue_body(mg_system* s, const NhConst& C, Buffers& b, cudaGraphConditiona
     const Dev& d = system_dev(s);
     int rows = 0;
     MCHK(system_enqueue_force(s, 0, 0, &rows));  // f and rho were zeroed by k_md_center
-    k_md_kick2<<<C.nblocks_own, kMdBlock, 0, st>>>(d, C, b.S, b.xd, b.part);
-    k_md_kick_drift<<<C.nblocks_own, kMdBlock, 0, st>>>(d, C, b.S, b.xd, b.xu, b.part);
-    k_md_center<<<C.nblocks_all, kMdBlock, 0, st>>>(d, C, b.S, b.xu, h, 1);
+    launch_dep(k_md_kick2, C.nblocks_own, kMdBlock, 0, st, d, C, b.S, b.xd, b.part);
+    launch_dep(k_md_kick_drift, C.nblocks_own, kMdBlock, 0, st, d, C, b.S, b.xd, b.xu, b.part);
+    launch_dep(k_md_center, C.nblocks_all, kMdBlock, 0, st, d, C, b.S, b.xu, h, 1);
     MCU(cudaGetLastError());
     return MG_OK;
 }
@@ -517,9 +523,9 @@ extern "C" int mg_md_nh(mg_system* s, double t_tar, double t_period, int eta_ite
         {
             const Dev& d = system_dev(s);
             C.nblocks_all = div_up((long long)d.natms + d.nph, kMdBlock);
-            k_md_begin<<<1, 32, 0, st>>>(b.S, C);
-            k_md_kick_drift<<<C.nblocks_own, kMdBlock, 0, st>>>(d, C, b.S, b.xd, b.xu, b.part);
-            k_md_center<<<C.nblocks_all, kMdBlock, 0, st>>>(d, C, b.S, b.xu, cudaGraphConditionalHandle{}, 0);
+            launch_dep(k_md_begin, 1, 32, 0, st, b.S, C);
+            launch_dep(k_md_kick_drift, C.nblocks_own, kMdBlock, 0, st, d, C, b.S, b.xd, b.xu, b.part);
+            launch_dep(k_md_center, C.nblocks_all, kMdBlock, 0, st, d, C, b.S, b.xu, cudaGraphConditionalHandle{}, 0);
             MCU(cudaGetLastError());
         }
         bool need_capture = true;
@@ -544,7 +550,7 @@ extern "C" int mg_md_nh(mg_system* s, double t_tar, double t_period, int eta_ite
             }
             MCU(cudaGraphLaunch(b.exec, st));
         }
-        k_md_finish<<<C.nblocks_own, kMdBlock, 0, st>>>(system_dev(s), b.S, b.xd);
+        launch_dep(k_md_finish, C.nblocks_own, kMdBlock, 0, st, system_dev(s), b.S, b.xd);
         MCU(cudaGetLastError());
         // the thermo pass of the last step: force_calc(1) at the final positions
         MCHK(system_enqueue_force(s, 1, 1, &rows));

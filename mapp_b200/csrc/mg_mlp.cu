@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 #include "mg_dmd_common.cuh"
 #include "mg_mlp_common.cuh"
 
@@ -236,14 +237,6 @@ struct TrainTile {
     float b[3][H], b4[8], loss[4];
 };
 
-// Programmatic dependent launch: a step's two kernels are queued with
-// overlapping starts.  dep_start lets the next kernel's blocks be scheduled,
-// dep_wait returns when everything before this kernel in the stream is complete
-// and visible; what runs before it (the rows of a training tile) depends on
-// nothing the previous kernel writes.
-__device__ __forceinline__ void dep_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p)
 {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -318,7 +311,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpState S, const f
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainTile& T = *reinterpret_cast<TrainTile*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    dep_start();
+    dep_start();  // (before dep_wait: the rows of a tile depend on nothing the previous step writes)
     // 8 threads per row: one takes the inputs, six a target each
     if (tid < kRows * 8) {
         const int r = tid >> 3, part = tid & 7;
@@ -575,22 +568,10 @@ cudaError_t launch_mlp_train_step(const MlpState& S, const float* X, const float
         if (e != cudaSuccess) return e;
     }
     int nb = batch / kRows;
-    cudaLaunchAttribute dep;
-    dep.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    dep.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(kTrainThreads);
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
-    cfg.attrs = &dep;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_mlp_train, S, X, Y, n, batch, seed, step, fixed);
+    cudaError_t e = launch_dep(k_mlp_train, nb, kTrainThreads, sm, st, S, X, Y, n, batch, seed, step, fixed);
     if (e != cudaSuccess) return e;
-    cfg.gridDim = dim3(div_up(NPARAM + 1, kAdamThreads));
-    cfg.blockDim = dim3(kAdamThreads);
-    cfg.dynamicSmemBytes = 0;
-    e = cudaLaunchKernelEx(&cfg, k_mlp_adam, S, nb, step, total, lr, grad_out, loss_hist);
+    e = launch_dep(k_mlp_adam, div_up(NPARAM + 1, kAdamThreads), kAdamThreads, 0, st, S, nb, step, total, lr, grad_out,
+                   loss_hist);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -34,6 +34,7 @@
 // Every wait on the tensor core is bounded (200 ms of %globaltimer); a wait
 // that runs out sets status[5], frees the CTA's TMEM and ends the CTA.
 #include "mg_reduce.cuh"
+#include "mg_launch.cuh"
 #include "mg_dmd_common.cuh"
 #include "mg_mlp_common.cuh"
 #include "mg_split.cuh"
@@ -300,6 +301,7 @@ __device__ __forceinline__ bool audited(unsigned long long seed, long long p, in
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock) k_mlp_rows(Dev d, MlpState S, unsigned long long audit_seed)
 {
+    dep_sync();
     using SL = Slots<NT>;
     constexpr int RP = NT * NT;
     __shared__ int warp_n[kFFWarps];
@@ -433,6 +435,7 @@ __global__ void __launch_bounds__(kFFBlock) k_mlp_rows(Dev d, MlpState S, unsign
 template <int NT, int NQ>
 __global__ void __launch_bounds__(kFFBlock) k_mlp_fallback(Dev d, MlpState S)
 {
+    dep_sync();
     // the split table in shared memory, as the precision form's force pass has it
     extern __shared__ float4 tab[];
     load_split_table(d, tab, NT * NT + Slots<NT>::NC);
@@ -485,6 +488,7 @@ __global__ void __launch_bounds__(kFFBlock) k_mlp_fallback(Dev d, MlpState S)
 template <int NT, int ACT>
 __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_tc(Dev d, MlpState S)
 {
+    dep_sync();
     extern __shared__ __align__(1024) unsigned char smraw[];
     TcSmem& T = *reinterpret_cast<TcSmem*>(smraw);
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -608,6 +612,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_tc(Dev d, MlpState S)
 template <int NT, int NQ>
 __global__ void __launch_bounds__(kFFBlock) k_mlp_audit(Dev d, MlpState S)
 {
+    dep_sync();
     using SL = Slots<NT>;
     const int lane = threadIdx.x & 31;
     const F32Consts kc = f32_consts(d);
@@ -655,6 +660,7 @@ __global__ void __launch_bounds__(kFFBlock) k_mlp_audit(Dev d, MlpState S)
 template <int NT>
 __global__ void __launch_bounds__(kFFBlock, 4) k_mlp_densities(Dev d, int row0)
 {
+    dep_sync();
     using SL = Slots<NT>;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -743,19 +749,19 @@ cudaError_t mlp_force_nt(const Dev& d, const MlpState& S, unsigned long long aud
     cudaError_t e = cudaMemsetAsync(S.row_n, 0, 4 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     if (evs) cudaEventRecord(evs[0], st);
-    k_mlp_rows<NT><<<std::max(g0, 1), kFFBlock, 0, st>>>(d, S, audit_seed);
+    launch_dep(k_mlp_rows<NT>, std::max(g0, 1), kFFBlock, 0, st, d, S, audit_seed);
     const size_t smF = (size_t)(NT * NT + NT * (NT + 1) / 2) * d.nrS * sizeof(float4);
     if (smF > 48 * 1024) {
         e = cudaFuncSetAttribute(nq3 ? k_mlp_fallback<NT, 3> : k_mlp_fallback<NT, 0>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smF);
         if (e != cudaSuccess) return e;
     }
-    if (nq3) k_mlp_fallback<NT, 3><<<num_sms() * 4, kFFBlock, smF, st>>>(d, S);
-    else k_mlp_fallback<NT, 0><<<num_sms() * 4, kFFBlock, smF, st>>>(d, S);
-    k_mlp_tc<NT, ACT><<<g1, kTcThreads, sm, st>>>(d, S);
-    if (d.nq == 3) k_mlp_audit<NT, 3><<<num_sms(), kFFBlock, 0, st>>>(d, S);
-    else k_mlp_audit<NT, 0><<<num_sms(), kFFBlock, 0, st>>>(d, S);
-    k_mlp_densities<NT><<<gd, kFFBlock, 0, st>>>(d, 0);
+    if (nq3) launch_dep(k_mlp_fallback<NT, 3>, num_sms() * 4, kFFBlock, smF, st, d, S);
+    else launch_dep(k_mlp_fallback<NT, 0>, num_sms() * 4, kFFBlock, smF, st, d, S);
+    launch_dep(k_mlp_tc<NT, ACT>, g1, kTcThreads, sm, st, d, S);
+    if (d.nq == 3) launch_dep(k_mlp_audit<NT, 3>, num_sms(), kFFBlock, 0, st, d, S);
+    else launch_dep(k_mlp_audit<NT, 0>, num_sms(), kFFBlock, 0, st, d, S);
+    launch_dep(k_mlp_densities<NT>, gd, kFFBlock, 0, st, d, 0);
     if (evs) cudaEventRecord(evs[1], st);
     int rows = 0;
     e = launch_dmd_force_f32_after_pass1(d, st_clc, gd, &rows, st, evs);
