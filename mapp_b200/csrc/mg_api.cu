@@ -252,7 +252,7 @@ struct mg_system {
     struct HostPin {
         double tot[8];
         int status[8];
-        GhostCtl gc;
+        RebuildOut rb;
         int count;
     };
     HostPin* hp = nullptr;
@@ -285,10 +285,13 @@ struct mg_system {
     // the value update_x's skin test writes to status[7] when some site moved
     // more than the skin: a new one per update_x, so the word needs no reset
     int skin_gen = 0;
+    RebuildOut* rb_out = nullptr;
     GhostCtl* gctl = nullptr;  // device control of the ghost passes (two, ping-pong)
     unsigned* gtiles = nullptr;  // look-back words of the ghost passes (two halves)
     int gtiles_cap = 0;
-    double t_list = 0, t_force = 0, t_energy = 0, t_cd = 0, t_g = 0;
+    cudaEvent_t ev_l0 = nullptr, ev_l1 = nullptr;  // around the last list build
+    bool list_timed = false;
+    double t_force = 0, t_energy = 0, t_cd = 0, t_g = 0;
     double t_k[3] = {0, 0, 0};  // DMD force: pass 1, embedding, pass 2
     long long partial_rows = 0;
     bool tables_uploaded = false;  // device tables match the last ff_coef
@@ -553,39 +556,20 @@ int rebuild(mg_system* s)
 {
     Dev& d = s->d;
     cudaStream_t st = s->st;
-    CU(cudaEventRecord(s->ev0, st));
+    CU(cudaEventRecord(s->ev_l0, st));
     int natms = s->natms, nph = 0;
     fill_dev_scalars(s);
     if (!s->gctl) CHK(dalloc(&s->gctl, 2));
-    // The ghost passes run back to back on the device (bounds and counts in
-    // GhostCtl, one launch per pass), and so do binning and the half list,
-    // which read the ghost count from the device. One synchronisation reads
+    if (!s->rb_out) CHK(dalloc(&s->rb_out, 1));
+    // The ghost passes run on the device (one cluster launch, or one launch per
+    // pass with bounds and counts in GhostCtl), and so do binning and the half
+    // list, which read the ghost count from the device. One synchronisation reads
     // the ghost count, the list's overflow word and the pair count; ghosts that
     // did not fit the arrays make them grow and the build run again, a list
     // overflow makes the per-atom list capacity grow and the list run again.
     int np_h = 0;
     for (int attempt = 0;; attempt++) {
         const int cap = (int)s->cap, nt_tiles = ghost_tiles(cap);
-        // the tile words of both halves, then the two tickets: one memset
-        if (2 * nt_tiles + 2 > s->gtiles_cap) {
-            CHK(dalloc(&s->gtiles, (size_t)2 * nt_tiles + 2));
-            s->gtiles_cap = 2 * nt_tiles + 2;
-        }
-        int* gticket = reinterpret_cast<int*>(s->gtiles + 2 * nt_tiles);
-        CU(cudaMemsetAsync(d.status, 0, 8 * sizeof(int), st));
-        CU(cudaMemsetAsync(s->gtiles, 0, ((size_t)2 * nt_tiles + 2) * sizeof(unsigned), st));
-        CU(launch_ghost_init(d, s->gctl, st));
-        int cur = 0;
-        for (int dim = 0; dim < 3; dim++)
-            for (int dir = 0; dir < 2; dir++)
-                for (int pass = 0; pass < s->comm_need[dim]; pass++) {
-                    const int next_mode = pass + 1 < s->comm_need[dim] ? 0 : (dir == 0 ? 1 : 2);
-                    CU(launch_ghost_pass(d, s->gctl + cur, s->gctl + (cur ^ 1), s->gtiles + cur * nt_tiles,
-                                         s->gtiles + (cur ^ 1) * nt_tiles, gticket + cur, gticket + (cur ^ 1),
-                                         cap, dim, dir, next_mode, st));
-                    cur ^= 1;
-                }
-        const GhostCtl* gfin = s->gctl + cur;
         // bins
         if (d.tot_bin + 1 > s->cap_bins) {
             CHK(dalloc(&d.cell_count, 2 * ((size_t)d.tot_bin + 1)));
@@ -598,26 +582,50 @@ int rebuild(mg_system* s)
             }
         }
         // the fill cursors sit right after this build's counts (the allocation
-        // holds two arrays of cap_bins), so one memset zeroes both
+        // holds two arrays of cap_bins), so both are cleared together
         s->cursor = d.cell_count + d.tot_bin + 1;
-        CU(cudaMemsetAsync(d.cell_count, 0, 2 * ((size_t)d.tot_bin + 1) * sizeof(int), st));
+        const GhostCtl* gfin = s->gctl;
+        if (ghosts_by_cluster(natms)) {
+            CU(launch_ghost_cluster(d, s->gctl, cap, s->comm_need, d.cell_count, 2 * (d.tot_bin + 1), st));
+        } else {
+            // the tile words of both halves, then the two tickets: one memset
+            if (2 * nt_tiles + 2 > s->gtiles_cap) {
+                CHK(dalloc(&s->gtiles, (size_t)2 * nt_tiles + 2));
+                s->gtiles_cap = 2 * nt_tiles + 2;
+            }
+            int* gticket = reinterpret_cast<int*>(s->gtiles + 2 * nt_tiles);
+            CU(cudaMemsetAsync(d.status, 0, 8 * sizeof(int), st));
+            CU(cudaMemsetAsync(s->gtiles, 0, ((size_t)2 * nt_tiles + 2) * sizeof(unsigned), st));
+            CU(launch_ghost_init(d, s->gctl, st));
+            int cur = 0;
+            for (int dim = 0; dim < 3; dim++)
+                for (int dir = 0; dir < 2; dir++)
+                    for (int pass = 0; pass < s->comm_need[dim]; pass++) {
+                        const int next_mode = pass + 1 < s->comm_need[dim] ? 0 : (dir == 0 ? 1 : 2);
+                        CU(launch_ghost_pass(d, s->gctl + cur, s->gctl + (cur ^ 1), s->gtiles + cur * nt_tiles,
+                                             s->gtiles + (cur ^ 1) * nt_tiles, gticket + cur, gticket + (cur ^ 1),
+                                             cap, dim, dir, next_mode, st));
+                        cur ^= 1;
+                    }
+            gfin = s->gctl + cur;
+            CU(cudaMemsetAsync(d.cell_count, 0, 2 * ((size_t)d.tot_bin + 1) * sizeof(int), st));
+        }
         CU(launch_bin_and_s2x(d, gfin, cap, st));
         CU(launch_exclusive_scan(d.cell_count, d.cell_start, d.tot_bin + 1, s->scan_tmp, s->scan_tmp_bytes, st));
         CU(launch_cell_fill(d, s->cursor, gfin, cap, st));
         // half list, then the scan of the per-atom counts
         bool regrow_ghosts = false;
         for (int attempt_nb = 0;; attempt_nb++) {
-            const GhostCtl& gc = s->hp->gc;
-            const int* st_h = s->hp->status;
+            const GhostCtl& gc = s->hp->rb.gc;
+            const int* st_h = s->hp->rb.status;
             // (the list kernel zeroes nnb[natms], the scan's last element)
             if (attempt_nb) CU(cudaMemsetAsync(d.status, 0, 2 * sizeof(int), st));
             CU(launch_neigh(d, st));
-            CU(launch_exclusive_scan(d.nnb, d.poff, natms + 1, s->scan_tmp, s->scan_tmp_bytes, st));
-            CU(cudaMemcpyAsync(&s->hp->gc, gfin, sizeof(GhostCtl), cudaMemcpyDeviceToHost, st));
-            CU(cudaMemcpyAsync(s->hp->status, d.status, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
-            CU(cudaMemcpyAsync(&s->hp->count, d.poff + natms, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CU(launch_exclusive_scan(d.nnb, d.poff, natms + 1, s->scan_tmp, s->scan_tmp_bytes, st, gfin, d.status,
+                                     s->rb_out));
+            CU(cudaMemcpyAsync(&s->hp->rb, s->rb_out, sizeof(RebuildOut), cudaMemcpyDeviceToHost, st));
             CU(cudaStreamSynchronize(st));
-            np_h = s->hp->count;
+            np_h = s->hp->rb.count;
             if (st_h[4])
                 return fail(MG_ERR_CAPACITY, "ghost image chain deeper than %d swaps (box too small for the cut-off)",
                             kMaxChain);
@@ -648,11 +656,8 @@ int rebuild(mg_system* s)
     CU(launch_pairs_compact(d, st));
     CU(launch_store_x0(d, st));
     s->crd_built = 0;
-    CU(cudaEventRecord(s->ev1, st));
-    CU(cudaEventSynchronize(s->ev1));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, s->ev0, s->ev1);
-    s->t_list = ms;
+    CU(cudaEventRecord(s->ev_l1, st));  // (read by mg_last_time, so that the host does not wait here)
+    s->list_timed = true;
     return MG_OK;
 }
 
@@ -1090,6 +1095,8 @@ int mg_create(const char* style, int device, mg_system** out)
     s->own_stream = true;
     cudaEventCreate(&s->ev0);
     cudaEventCreate(&s->ev1);
+    cudaEventCreate(&s->ev_l0);
+    cudaEventCreate(&s->ev_l1);
     for (int k = 0; k < 4; k++) cudaEventCreate(&s->evk[k]);
     memset(&s->d, 0, sizeof(Dev));
     int r = MG_OK;
@@ -1114,6 +1121,8 @@ int mg_create(const char* style, int device, mg_system** out)
         for (int k = 0; k < 4; k++) cudaEventDestroy(s->evk[k]);
         cudaEventDestroy(s->ev0);
         cudaEventDestroy(s->ev1);
+        cudaEventDestroy(s->ev_l0);
+        cudaEventDestroy(s->ev_l1);
         if (s->ev_fork) cudaEventDestroy(s->ev_fork);
         if (s->ev_join) cudaEventDestroy(s->ev_join);
         if (s->side) cudaStreamDestroy(s->side);
@@ -1135,7 +1144,7 @@ int mg_destroy(mg_system* s)
     void* ptrs[] = {d.prf, s->d_pkT, s->d_pk64, s->d_pkS, d.icut, d.icut_n, d.srec, d.dE32, d.facc, d.poff, d.pair_i, d.pair_j, d.pos, d.sfr, d.pos0, d.alpha, d.c, d.type, d.root, d.gchain, d.bin, d.cell_start,
                     d.cell_count, d.cell_pos, d.nbr, d.nnb, d.crdl, d.ncrd, d.crd, d.f, d.rho, d.E,
                     d.dE, d.ddE, d.n, d.s, d.t, d.v, d.c_d, d.a_in, d.g, d.pr, d.partial, d.act_pj, d.act_pv, d.act_off, d.nact,
-                    s->scan_tmp, s->stage, s->red_out, s->d_rhoT, s->d_phiT, s->d_FT, s->gctl, s->gtiles};
+                    s->scan_tmp, s->stage, s->red_out, s->d_rhoT, s->d_phiT, s->d_FT, s->gctl, s->gtiles, s->rb_out};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* mptrs[] = {s->mlp.par, s->mlp.wbf, s->mlp.m, s->mlp.v, s->mlp.gpart, s->mlp.audit, s->mlp_loss,
@@ -1144,6 +1153,8 @@ int mg_destroy(mg_system* s)
         if (p) cudaFree(p);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
+    if (s->ev_l0) cudaEventDestroy(s->ev_l0);
+    if (s->ev_l1) cudaEventDestroy(s->ev_l1);
     for (int k = 0; k < 4; k++)
         if (s->evk[k]) cudaEventDestroy(s->evk[k]);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);
@@ -1778,7 +1789,15 @@ int mg_last_time(mg_system* s, const char* phase, double* ms)
 {
     CHK(check_sys(s));
     if (!phase || !ms) return fail(MG_ERR_ARG, "null argument");
-    if (!strcmp(phase, "list")) *ms = s->t_list;
+    if (!strcmp(phase, "list")) {
+        *ms = 0.0;
+        if (s->list_timed) {
+            float t = 0;
+            CU(cudaEventSynchronize(s->ev_l1));
+            CU(cudaEventElapsedTime(&t, s->ev_l0, s->ev_l1));
+            *ms = t;
+        }
+    }
     else if (!strcmp(phase, "force")) *ms = s->t_force;
     else if (!strcmp(phase, "energy")) *ms = s->t_energy;
     else if (!strcmp(phase, "c_d")) *ms = s->t_cd;

@@ -8,6 +8,7 @@
 // s2bin neighbor.cpp:507-525, rsq neighbor.cpp:212-215, ghost s shift
 // atoms.cpp:489-495, ghost x refresh atoms.cpp:1340-1348, skin check
 // atoms.cpp:1804-1819.
+#include <cooperative_groups.h>
 #include <cub/device/device_scan.cuh>
 
 #include "mg_internal.h"
@@ -227,6 +228,217 @@ __global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* __
         else atomicExch(&d.status[4], 1);  // chain too deep: reported as a capacity error
         d.gchain[g] = ch;
     }
+}
+
+// The whole of Atoms::ph_setup for systems of up to kClusterSites sites: every
+// pass in one launch of one thread-block cluster, so that a pass costs two
+// cluster barriers instead of a kernel and its look-back chain (six launches, 66
+// us in all at 10000 and 32000 sites; this kernel takes 36 and 54 us, a whole list
+// build 172 -> 102 and 220 -> 149 us).  A pass is a stable
+// compaction: each CTA counts the flagged atoms of its stretch, the counts are
+// exchanged through distributed shared memory, and the stretch is scattered in
+// order.  A dimension that needs one swap pass per direction (every box longer
+// than the cut-off) does both directions at once: the low shell's ghosts, then
+// the high shell's, over the same atoms.  Above kClusterSites the passes want
+// more SMs than a cluster has (42592 sites: 198 us a build by passes, 204 us by
+// the cluster; 108000: 320 and 395).  zero[0..nzero) is the list build's counters,
+// cleared here as well as the status words.
+constexpr int kClusterSites = 40000, kClusterThreads = 1024;
+
+__global__ void __launch_bounds__(kClusterThreads) k_ghost_cluster(Dev d, GhostCtl* __restrict__ out, int cap, int need0,
+                                                                   int need1, int need2, int* __restrict__ zero, int nzero)
+{
+    dep_sync();
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ int s_cnt[2], s_all[2][16], s_w[2][32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int CS = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const unsigned lt = (1u << lane) - 1u;
+    for (int k = rank * kClusterThreads + tid; k < nzero; k += CS * kClusterThreads) zero[k] = 0;
+    if (rank == 0 && tid < 8) d.status[tid] = 0;
+    cl.sync();
+    int nph = 0, over = 0;
+    // arrays that earlier passes of other CTAs wrote are read from L2
+    auto flags = [&](int k, int dim, int mask) {
+        const double sv = __ldcg(reinterpret_cast<const double*>(d.sfr + k) + dim);
+        return ((mask & 1) && sv <= d.s_ph_lo[dim] ? 1 : 0) | ((mask & 2) && d.s_ph_hi[dim] <= sv ? 2 : 0);
+    };
+    auto emit = [&](int src, int g, int dim, int dir) {
+        if (g >= cap) return;
+        // every load first: one round trip to L2, not one per array
+        const double2* sp = reinterpret_cast<const double2*>(d.sfr + src);
+        const double2 u = __ldcg(sp), v = __ldcg(sp + 1);
+        double al[kMaxTypes], cc[kMaxTypes];
+#pragma unroll
+        for (int a = 0; a < kMaxTypes; a++) {
+            if (a < d.x_dim - 3) al[a] = __ldcg(d.alpha + (size_t)src * d.nt + a);
+            if (d.c && a < d.nt) cc[a] = __ldcg(d.c + (size_t)src * d.nt + a);
+        }
+        const int ty = d.type ? __ldcg(d.type + src) : 0, ro = __ldcg(d.root + src);
+        unsigned long long ch = __ldcg(d.gchain + src);
+        double4 s = make_double4(u.x, u.y, v.x, v.y);
+        const double x = comp3(s, dim);
+        set3(s, dim, dir == 0 ? dadd(x, 1.0) : dsub(x, 1.0));
+        d.sfr[g] = s;
+#pragma unroll
+        for (int a = 0; a < kMaxTypes; a++) {
+            if (a < d.x_dim - 3) d.alpha[(size_t)g * d.nt + a] = al[a];
+            if (d.c && a < d.nt) d.c[(size_t)g * d.nt + a] = cc[a];
+        }
+        if (d.type) d.type[g] = ty;
+        d.root[g] = ro;
+        const int used = __popcll(ch & 0x8888888888888888ull);
+        if (used < kMaxChain) ch |= (unsigned long long)(8 | (dim << 1) | dir) << (4 * used);
+        else atomicExch(&d.status[4], 1);  // chain too deep: reported as a capacity error
+        d.gchain[g] = ch;
+    };
+    // the atoms of [lo, hi) in the shells of mask (1 low, 2 high) appended in order
+    auto pass = [&](int lo, int hi, int dim, int mask) {
+        const int n = max(min(hi, cap) - lo, 0);
+        const int per = ((n + CS - 1) / CS + 31) & ~31;
+        const int a = lo + min(rank * per, n), e = lo + min((rank + 1) * per, n);
+        int c0 = 0, c1 = 0;
+        for (int k = a + tid; k < e; k += kClusterThreads) {
+            const int f = flags(k, dim, mask);
+            c0 += f & 1;
+            c1 += f >> 1;
+        }
+        c0 = __reduce_add_sync(0xffffffffu, c0);
+        c1 = __reduce_add_sync(0xffffffffu, c1);
+        if (lane == 0) {
+            s_w[0][w] = c0;
+            s_w[1][w] = c1;
+        }
+        __syncthreads();
+        if (w < 2) {
+            const int t = __reduce_add_sync(0xffffffffu, s_w[w][lane]);
+            if (lane == 0) s_cnt[w] = t;
+        }
+        cl.sync();
+        if (tid < 2 * CS) {
+            const int r = tid >> 1, q = tid & 1;
+            s_all[q][r] = *cl.map_shared_rank(&s_cnt[q], r);
+        }
+        __syncthreads();
+        int ex[2] = {0, 0}, tot[2] = {0, 0};
+        for (int r = 0; r < CS; r++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int v = s_all[q][r];
+                ex[q] += r < rank ? v : 0;
+                tot[q] += v;
+            }
+        const int base = d.natms + nph;
+        int run[2] = {base + ex[0], base + tot[0] + ex[1]};
+        for (int k0 = a; k0 < e; k0 += kClusterThreads) {
+            const int k = k0 + tid;
+            const int f = k < e ? flags(k, dim, mask) : 0;
+            const unsigned m0 = __ballot_sync(0xffffffffu, f & 1), m1 = __ballot_sync(0xffffffffu, f & 2);
+            if (lane == 0) {
+                s_w[0][w] = __popc(m0);
+                s_w[1][w] = __popc(m1);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int v = s_w[q][lane];
+                const int before = __reduce_add_sync(0xffffffffu, lane < w ? v : 0);
+                const int all = __reduce_add_sync(0xffffffffu, v);
+                if (f >> q & 1) emit(k, run[q] + before + __popc((q ? m1 : m0) & lt), dim, q);
+                run[q] += all;
+            }
+            __syncthreads();
+        }
+        nph += tot[0] + tot[1];
+        over = max(over, d.natms + nph - cap);
+        cl.sync();
+    };
+    const int need[3] = {need0, need1, need2};
+#pragma unroll
+    for (int dim = 0; dim < 3; dim++) {
+        const int hi_dim = d.natms + nph;
+        if (need[dim] == 1) {
+            pass(0, hi_dim, dim, 3);
+        } else {
+            for (int dir = 0; dir < 2; dir++) {
+                int lo = 0, hi = hi_dim;
+                for (int p = 0; p < need[dim]; p++) {
+                    const int made = d.natms + nph;
+                    pass(lo, hi, dim, 1 << dir);
+                    lo = made;
+                    hi = d.natms + nph;
+                }
+            }
+        }
+    }
+    if (rank == 0 && tid == 0) {
+        GhostCtl o;
+        o.lo = o.hi = o.hi_dim = 0;
+        o.nph = nph;
+        o.over = over;
+        *out = o;
+    }
+}
+
+// Exclusive scan of up to kScanSmall ints by one block (one launch; the general
+// scan takes two), 4 per thread and tile, the next tile's loads in flight.  With
+// rb set it also gathers what the host reads after a list build: the ghost
+// control, the status words and the total (the last output).
+constexpr int kScanSmall = 65536;
+
+__global__ void __launch_bounds__(1024) k_scan_small(const int* __restrict__ in, int* __restrict__ out, int n,
+                                                     const GhostCtl* __restrict__ gc, const int* __restrict__ status,
+                                                     RebuildOut* __restrict__ rb)
+{
+    dep_sync();
+    __shared__ int s_w[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    auto load = [&](int k) {
+        int4 v = make_int4(0, 0, 0, 0);
+        if (k + 3 < n) v = *reinterpret_cast<const int4*>(in + k);
+        else {
+            if (k < n) v.x = in[k];
+            if (k + 1 < n) v.y = in[k + 1];
+            if (k + 2 < n) v.z = in[k + 2];
+        }
+        return v;
+    };
+    int run = 0;
+    int4 v = load(4 * tid);
+    for (int b = 0; b < n; b += 4096) {
+        const int k = b + 4 * tid;
+        const int4 next = load(k + 4096);
+        const int sum = v.x + v.y + v.z + v.w;
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) s_w[w] = incl;
+        __syncthreads();
+        const int ws = s_w[lane];
+        const int before = __reduce_add_sync(0xffffffffu, lane < w ? ws : 0);
+        const int all = __reduce_add_sync(0xffffffffu, ws);
+        int4 o;
+        o.x = run + before + incl - sum;
+        o.y = o.x + v.x;
+        o.z = o.y + v.y;
+        o.w = o.z + v.z;
+        if (k + 3 < n) *reinterpret_cast<int4*>(out + k) = o;
+        else {
+            if (k < n) out[k] = o.x;
+            if (k + 1 < n) out[k + 1] = o.y;
+            if (k + 2 < n) out[k + 2] = o.z;
+        }
+        if (rb && k <= n - 1 && n - 1 <= k + 3) rb->count = n - 1 == k ? o.x : n - 1 == k + 1 ? o.y : n - 1 == k + 2 ? o.z : o.w;
+        run += all;
+        v = next;
+        __syncthreads();
+    }
+    if (rb && tid < 8) rb->status[tid] = status[tid];
+    if (rb && tid == 8) rb->gc = *gc;
 }
 
 __global__ void k_ghost_ctl_init(Dev d, GhostCtl* c)
@@ -511,6 +723,28 @@ cudaError_t launch_ghost_pass(const Dev& d, const GhostCtl* ctl, GhostCtl* next,
     return cudaGetLastError();
 }
 
+bool ghosts_by_cluster(int natms) { return natms <= kClusterSites; }
+
+cudaError_t launch_ghost_cluster(const Dev& d, GhostCtl* out, int cap, const int* need, int* zero, int nzero, cudaStream_t st)
+{
+    // a CTA per 4096 atoms (owned and ghost), 8 at most
+    int cs = 1;
+    while (cs < 8 && cs * 4096 < 2 * d.natms) cs *= 2;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cs);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k_ghost_cluster, d, out, cap, need[0], need[1], need[2], zero, nzero);
+}
+
 cudaError_t launch_bin_and_s2x(const Dev& d, const GhostCtl* gc, int cap, cudaStream_t st)
 {
     const int n = gc ? cap : d.nall;
@@ -581,9 +815,16 @@ size_t scan_temp_bytes(int n)
     return bytes;
 }
 
-cudaError_t launch_exclusive_scan(const int* in, int* out, int n, void* temp, size_t temp_bytes, cudaStream_t st)
+cudaError_t launch_exclusive_scan(const int* in, int* out, int n, void* temp, size_t temp_bytes, cudaStream_t st,
+                                  const GhostCtl* gc, const int* status, RebuildOut* rb)
 {
-    return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, in, out, n, st);
+    if (n <= kScanSmall) return launch_dep(k_scan_small, 1, 1024, 0, st, in, out, n, gc, status, rb);
+    const cudaError_t e = cub::DeviceScan::ExclusiveSum(temp, temp_bytes, in, out, n, st);
+    if (e != cudaSuccess || !rb) return e;
+    // what k_scan_small gathers
+    cudaMemcpyAsync(&rb->gc, gc, sizeof(GhostCtl), cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(rb->status, status, 8 * sizeof(int), cudaMemcpyDeviceToDevice, st);
+    return cudaMemcpyAsync(&rb->count, out + n - 1, sizeof(int), cudaMemcpyDeviceToDevice, st);
 }
 
 }  // namespace mg

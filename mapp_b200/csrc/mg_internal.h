@@ -239,7 +239,17 @@ cudaError_t launch_split_x(const Dev& d, const double* x_aos, int frac, cudaStre
 struct GhostCtl {
     int lo, hi, nph, hi_dim, over;
 };
+// what the host reads after a list build
+struct RebuildOut {
+    GhostCtl gc;
+    int status[8];
+    int count;  // listed pairs
+};
 cudaError_t launch_ghost_init(const Dev& d, GhostCtl* ctl, cudaStream_t st);
+// every ghost pass in one launch, for systems of up to some ten thousand sites
+// (need: swap passes per dimension); clears the status words and zero[0..nzero)
+bool ghosts_by_cluster(int natms);
+cudaError_t launch_ghost_cluster(const Dev& d, GhostCtl* out, int cap, const int* need, int* zero, int nzero, cudaStream_t st);
 // one ghost pass: tile words and tickets of this pass and of the next
 // (ping-pong halves, ghost_tiles(cap) words each)
 int ghost_tiles(int cap);
@@ -259,7 +269,9 @@ cudaError_t launch_reduce_partials(const Dev& d, int nblocks, int nvals, double*
 // zeroes a[0..na) and b[0..nb)
 cudaError_t launch_zero(double* a, size_t na, double* b, size_t nb, cudaStream_t st);
 size_t scan_temp_bytes(int n);
-cudaError_t launch_exclusive_scan(const int* in, int* out, int n, void* temp, size_t temp_bytes, cudaStream_t st);
+// (rb, when given: the ghost control, the status words and the last output, for the host)
+cudaError_t launch_exclusive_scan(const int* in, int* out, int n, void* temp, size_t temp_bytes, cudaStream_t st,
+                                  const GhostCtl* gc = nullptr, const int* status = nullptr, RebuildOut* rb = nullptr);
 // EAM / FS
 cudaError_t launch_eam_force(const Dev& d, int st_clc, int* nblocks_out, cudaStream_t st);
 cudaError_t launch_eam_energy(const Dev& d, int* nblocks_out, cudaStream_t st);
