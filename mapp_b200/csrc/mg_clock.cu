@@ -41,6 +41,8 @@ struct CkView {
     double* c;      // owned then ghost concentrations (the system's)
     const double* c_d;
     const double* g;
+    const double* s;  // calc_g's s, whose squares are the cost
+    double* E;        // calc_g's densities, cleared before every call
     double* a;      // calc_g's input (the system's a_in)
     double* g0;
     double* c0;
@@ -157,24 +159,6 @@ __global__ void __launch_bounds__(kCkBlock) k_ck_predict(CkView V, double dt)
     if (i >= V.n) return;
     const double r = V.sc[SC_RATIO];
     V.c[i] = dadd(V.c[i], dmul(dmul(V.c_d[i], dt), r));
-}
-
-// g.g0 and g.g after the line search (clock_adams.cpp:340-352)
-__global__ void __launch_bounds__(kCkBlock) k_ck_dots(CkView V)
-{
-    dep_sync();
-    const int i = blockIdx.x * kCkBlock + threadIdx.x;
-    double v[2] = {0.0, 0.0};
-    if (i < V.n) {
-        const double gi = V.g[i];
-        v[0] = dmul(gi, V.g0[i]);
-        v[1] = dmul(gi, gi);
-    }
-    double tot[2];
-    if (reduce_last<2, 0u>(v, V, tot) && threadIdx.x == 0) {
-        V.sc[SC_GG0] = tot[0];
-        V.sc[SC_GG] = tot[1];
-    }
 }
 
 // the first direction h = g with g.g, fused with the start of the first
@@ -403,35 +387,39 @@ __global__ void k_bs_init(SolveDev* S, const double* red_out, const double* sc, 
 }
 
 // the body's point: c0 + max_gamma h, or c0 itself after a failed line
-// search; ghosts from their owners (what the reference's refresh copies)
+// search; ghosts from their owners (what the reference's refresh copies).
+// calc_g's densities are cleared here, and a direction that restarts from g
+// (copy_hg) is written here.
 __global__ void __launch_bounds__(kCkBlock) k_bs_trial(CkView V, const SolveDev* S)
 {
     dep_sync();
-    if (S->mode == 2) return;  // the full calc_g at the last point
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
+    const bool copy = S->copy_hg != 0, full = S->mode == 2;  // full: calc_g at the last point
     const bool restore = S->mode == 1;
     const double gamma = S->max_gamma;
+    const double* h = copy ? V.g : V.h;
     if (i < V.n) {
-        V.c[i] = restore ? V.c0[i] : dadd(V.c0[i], dmul(gamma, V.h[i]));
+        V.E[i] = 0.0;
+        const double hi = h[i];
+        if (copy) V.h[i] = hi;
+        if (!full) V.c[i] = restore ? V.c0[i] : dadd(V.c0[i], dmul(gamma, hi));
         return;
     }
     const int k = i - V.n;
-    if (k >= V.nph * V.nt) return;
+    if (full || k >= V.nph * V.nt) return;
     const int gq = k / V.nt, a = k - gq * V.nt;
     const size_t o = (size_t)V.root[V.natms + gq] * V.nt + a;
-    V.c[(size_t)(V.natms + gq) * V.nt + a] = restore ? V.c0[o] : dadd(V.c0[o], dmul(gamma, V.h[o]));
+    V.c[(size_t)(V.natms + gq) * V.nt + a] = restore ? V.c0[o] : dadd(V.c0[o], dmul(gamma, h[o]));
 }
 
 // the Armijo test of the body's calc_g and the step reduction
 // (clock_bdf.cpp:760-806)
-__global__ void k_bs_post(SolveDev* S, const double* red_out, const double* sc)
+__device__ void bs_post(SolveDev* S, double sum_s2, double g_g0, double g_g)
 {
-    dep_sync();
-    if (threadIdx.x) return;
     S->n_calc_g++;
-    S->curr_cost = dmul(red_out[0], 0.25);
-    S->g_g0 = sc[SC_GG0];
-    S->g_g = sc[SC_GG];
+    S->curr_cost = dmul(sum_s2, 0.25);
+    S->g_g0 = g_g0;
+    S->g_g = g_g;
     S->need_next = 0;
     S->line_done = 1;
     if (S->adams) {
@@ -475,14 +463,62 @@ __global__ void k_bs_post(SolveDev* S, const double* red_out, const double* sc)
     }
 }
 
+// g.g0, g.g (clock_adams.cpp:340-352) and the cost's sum s^2 after the body's
+// calc_g; the last block goes on with the Armijo test
+__global__ void __launch_bounds__(kCkBlock) k_bs_dots(CkView V, SolveDev* S)
+{
+    dep_sync();
+    const int i = blockIdx.x * kCkBlock + threadIdx.x;
+    double v[3] = {0.0, 0.0, 0.0};
+    if (i < V.n) {
+        const double gi = V.g[i], si = V.s[i];
+        v[0] = dmul(gi, V.g0[i]);
+        v[1] = dmul(gi, gi);
+        v[2] = dmul(si, si);
+    }
+    double tot[3];
+    if (reduce_last<3, 0u>(v, V, tot) && threadIdx.x == 0) bs_post(S, tot[2], tot[0], tot[1]);
+}
+
+// the end of an outer iteration: h.g, the step bounds, the restart from g
+// when h.g < 0 (clock_bdf.cpp:810-828; the next trial point copies it), then the
+// outer loop's test.  gh, bound, bound_g: of the updated direction, when there is one.
+__device__ void bs_fin(SolveDev* S, double gh, double bound, double bound_g, cudaGraphConditionalHandle h)
+{
+    bool go = true;
+    S->copy_hg = 0;
+    if (S->line_done) {
+        if (S->need_next) {
+            S->g_h = gh;
+            S->bound = bound;
+            if (S->g_h < 0.0) {
+                S->copy_hg = 1;
+                S->g_h = S->g_g;
+                S->bound = bound_g;
+            }
+        }
+        S->iter++;
+        go = bs_outer_top(*S);
+    }
+    if (go && S->n_calc_g >= kBsGuard) {
+        S->overrun = 1;
+        go = false;
+    }
+    cudaGraphSetConditional(h, go ? 1u : 0u);
+}
+
 // the direction update h = h ratio + g with h.g (clock_adams.cpp:356-366,
 // clock_bdf.cpp:810-828), fused with the start of the next iteration: g0 = g,
 // c0 = c, and the box bounds along the new h and along g (the direction
-// restarts from g when h.g < 0); only when the body's post step asked for it
-__global__ void __launch_bounds__(kCkBlock) k_bs_next_dir(CkView V, const SolveDev* S)
+// restarts from g when h.g < 0); only when the body's Armijo test asked for it.
+// The last block (the first, without an update) ends the iteration.
+__global__ void __launch_bounds__(kCkBlock) k_bs_next_dir(CkView V, SolveDev* S, cudaGraphConditionalHandle h)
 {
     dep_sync();
-    if (!S->need_next) return;
+    if (!S->need_next) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) bs_fin(S, 0.0, 0.0, 0.0, h);
+        return;
+    }
     const double ratio = S->ratio;
     const int i = blockIdx.x * kCkBlock + threadIdx.x;
     double v[3] = {0.0, 1.0, 1.0};
@@ -497,47 +533,7 @@ __global__ void __launch_bounds__(kCkBlock) k_bs_next_dir(CkView V, const SolveD
         v[2] = box_bound(ci, dadd(ci, gi), 1.0);
     }
     double tot[3];
-    if (reduce_last<3, 6u>(v, V, tot) && threadIdx.x == 0) {
-        V.sc[SC_GH] = tot[0];
-        V.sc[SC_GAMMA] = tot[1];
-        V.sc[SC_B] = tot[2];
-    }
-}
-
-// the end of an outer iteration: h.g, the step bounds, the restart from g
-// when h.g < 0 (clock_bdf.cpp:810-828), then the outer loop's test
-__global__ void k_bs_fin(SolveDev* S, const double* sc, cudaGraphConditionalHandle h)
-{
-    dep_sync();
-    if (threadIdx.x) return;
-    bool go = true;
-    S->copy_hg = 0;
-    if (S->line_done) {
-        if (S->need_next) {
-            S->g_h = sc[SC_GH];
-            S->bound = sc[SC_GAMMA];
-            if (S->g_h < 0.0) {
-                S->copy_hg = 1;
-                S->g_h = S->g_g;
-                S->bound = sc[SC_B];
-            }
-        }
-        S->iter++;
-        go = bs_outer_top(*S);
-    }
-    if (go && S->n_calc_g >= kBsGuard) {
-        S->overrun = 1;
-        go = false;
-    }
-    cudaGraphSetConditional(h, go ? 1u : 0u);
-}
-
-__global__ void __launch_bounds__(kCkBlock) k_bs_copy(CkView V, const SolveDev* S)
-{
-    dep_sync();
-    if (!S->copy_hg) return;
-    const int i = blockIdx.x * kCkBlock + threadIdx.x;
-    if (i < V.n) V.h[i] = V.g[i];
+    if (reduce_last<3, 6u>(v, V, tot) && threadIdx.x == 0) bs_fin(S, tot[0], tot[1], tot[2], h);
 }
 
 constexpr double kBeta[6][6] = {
@@ -605,18 +601,14 @@ struct Clock {
     {
         launch_dep(k_bs_trial, trial_grid(), kCkBlock, 0, st, V, S_dev);
         KCU(cudaGetLastError());
-        int rows = 0;
-        KCHK(system_enqueue_calc_g_dev(s, &S_dev->calc_chk, &S_dev->alpha, &rows));
-        launch_dep(k_ck_dots, grid(), kCkBlock, 0, st, V);
-        launch_dep(k_bs_post, 1, 32, 0, st, S_dev, system_red_out(s), V.sc);
-        launch_dep(k_bs_next_dir, grid(), kCkBlock, 0, st, V, S_dev);
-        launch_dep(k_bs_fin, 1, 32, 0, st, S_dev, V.sc, h);
-        launch_dep(k_bs_copy, grid(), kCkBlock, 0, st, V, S_dev);
+        KCHK(system_enqueue_calc_g_dev(s, &S_dev->calc_chk, &S_dev->alpha));
+        launch_dep(k_bs_dots, grid(), kCkBlock, 0, st, V, S_dev);
+        launch_dep(k_bs_next_dir, grid(), kCkBlock, 0, st, V, S_dev, h);
         KCU(cudaGetLastError());
         return MG_OK;
     }
 
-    // graph: k_bs_init, then WHILE (condition set by k_bs_init and k_bs_fin)
+    // graph: k_bs_init, then WHILE (condition set by k_bs_init and bs_fin)
     int build_ls_graph()
     {
         KCU(cudaMalloc(&S_dev, sizeof(SolveDev)));
@@ -972,6 +964,8 @@ extern "C" int mg_clock_adams(mg_system* s, int order, int nsteps, double delta_
     ck.V.c = d.c;
     ck.V.c_d = d.c_d;
     ck.V.g = d.g;
+    ck.V.s = d.s;
+    ck.V.E = d.E;
     ck.V.a = d.a_in;
     ck.V.g0 = ck.block;
     ck.V.c0 = ck.block + vec;
@@ -1067,6 +1061,8 @@ extern "C" int mg_clock_bdf(mg_system* s, int nsteps, const mg_bdf_opts* opts, d
     ck.V.c = d.c;
     ck.V.c_d = d.c_d;
     ck.V.g = d.g;
+    ck.V.s = d.s;
+    ck.V.E = d.E;
     ck.V.a = d.a_in;
     ck.V.g0 = ck.block;
     ck.V.c0 = ck.block + vec;

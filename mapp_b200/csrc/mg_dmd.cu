@@ -596,9 +596,11 @@ __global__ void __launch_bounds__(kFFBlock) k_cd_rates(Dev d)
     }
 }
 
-// calc_g: s = 2(c + a) then the rate terms (ff_dmd_I.cpp:2537-2564,
-// ff_dmd_II.cpp:2471-2511); block partial of sum s^2 computed in k_g_cost.
-// (with calc_g's finalisation of n, which needs nothing from other sites)
+// calc_g: s = 2(c + a), to which the rate terms are added (ff_dmd_I.cpp:2537-2564,
+// ff_dmd_II.cpp:2471-2511), with calc_g's finalisation of n, which needs nothing
+// from other sites, and g, t and v cleared (g stays zero in a cost-only call, as
+// the reference's does: cleared at ff_dmd_I.cpp:2444-2445, return before the g
+// terms)
 template <int NT>
 __global__ void k_g_sinit(Dev d, int mode)
 {
@@ -608,6 +610,9 @@ __global__ void k_g_sinit(Dev d, int mode)
     mu_nfinal<NT>(d, idx, mode);
     d.s[idx] = 2.0 * (d.c[idx] + d.a_in[idx]);
     if (d.style == STYLE_DMD_II) d.c_d[idx] = 0.0;
+    d.g[idx] = 0.0;
+    d.t[idx] = 0.0;
+    d.v[idx] = 0.0;
 }
 
 template <int NT, int G>
@@ -654,36 +659,28 @@ __global__ void __launch_bounds__(kFFBlock) k_g_srates(Dev d, double alpha)
     }
 }
 
-template <int NT>
-__global__ void __launch_bounds__(kFFBlock) k_g_cost(Dev d, int row0, int chk)
+// The cost, sum s^2 (block partials), then g = -s plus the first g terms, and t,
+// over the crd sub-list (ff_dmd_I.cpp:2566-2608, ff_dmd.cpp:2582-2605,
+// ff_dmd_II.cpp:2529-2564).
+template <int NT, int G>
+__global__ void __launch_bounds__(kFFBlock) k_g_trates(Dev d, double alpha, int chk, int row0)
 {
     dep_sync();
     if (d.g_chk) chk = *d.g_chk;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (idx < d.natms * NT) {
-        double s = d.s[idx];
-        acc[0] = s * s;
-        // the cost-only call leaves g zeroed, as the reference's does
-        // (g cleared at ff_dmd_I.cpp:2444-2445, return before the g terms)
-        d.g[idx] = chk ? 0.0 : -s;
-        d.t[idx] = 0.0;
-        d.v[idx] = 0.0;
-    }
-    block_partials<7>(acc, d.partial, row0 + blockIdx.x);
-}
-
-// t and the first g terms over the crd sub-list (ff_dmd_I.cpp:2582-2608,
-// ff_dmd.cpp:2582-2605, ff_dmd_II.cpp:2529-2564).
-template <int NT, int G>
-__global__ void __launch_bounds__(kFFBlock) k_g_trates(Dev d, double alpha)
-{
-    dep_sync();
-    if (d.g_chk && *d.g_chk) return;  // cost-only call: no g terms
     if (d.g_alpha) alpha = *d.g_alpha;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     int lane = threadIdx.x & (G - 1);
-    if (i >= d.natms) return;
+    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+    if (i < d.natms && lane == 0) {
+        double s[NT];
+#pragma unroll
+        for (int a = 0; a < NT; a++) {
+            s[a] = d.s[(size_t)i * NT + a];
+            acc[0] += s[a] * s[a];
+        }
+    }
+    block_partials<7>(acc, d.partial, row0 + blockIdx.x);
+    if (chk || i >= d.natms) return;  // cost-only call: no g terms
     double ni[NT], ci[NT], si[NT], ti[NT], gi[NT];
 #pragma unroll
     for (int a = 0; a < NT; a++) {
@@ -740,7 +737,7 @@ __global__ void __launch_bounds__(kFFBlock) k_g_trates(Dev d, double alpha)
         double s = group_sum<G>(ti[a]), g = group_sum<G>(gi[a]);
         if (lane == 0) {
             atomicAdd(&d.t[(size_t)i * NT + a], s);
-            atomicAdd(&d.g[(size_t)i * NT + a], g);
+            atomicAdd(&d.g[(size_t)i * NT + a], g - si[a]);
         }
     }
 }
@@ -969,10 +966,9 @@ cudaError_t dmd_calc_g_ntp(const Dev& d, int chk, double alpha, int* nb, cudaStr
     launch_dep(k_mu_npairs<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d);
     launch_dep(k_g_sinit<NT>, gs, kFFBlock, 0, st, d, d.style == STYLE_DMD_II ? 3 : 2);
     launch_dep(k_g_srates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d, alpha);
-    launch_dep(k_g_cost<NT>, gs, kFFBlock, 0, st, d, 0, chk);
-    *nb = gs;
+    launch_dep(k_g_trates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d, alpha, chk, 0);
+    *nb = gc;
     if (!chk || d.g_chk) {
-        launch_dep(k_g_trates<NT, kCrdLanes>, gc, kFFBlock, 0, st, d, alpha);
         launch_dep(k_g_vpass<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d, alpha);
         launch_dep(k_g_last<NT, P, kNbrLanes>, gw, kFFBlock, 0, st, d, alpha);
     }

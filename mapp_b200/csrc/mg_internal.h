@@ -358,8 +358,9 @@ double* system_red_out(mg_system* s);
 // g in the system's g unless chk) and c_d_calc's (c_d in the system's c_d); capturable
 int system_enqueue_calc_g(mg_system* s, int chk, double alpha, int* rows);
 // the same with chk and alpha read from device memory at run time (for a
-// captured loop whose iterations change them)
-int system_enqueue_calc_g_dev(mg_system* s, const int* chk_dev, const double* alpha_dev, int* rows);
+// captured loop whose iterations change them), without clearing the densities
+// before and without reducing the cost after: the loop's own kernels do
+int system_enqueue_calc_g_dev(mg_system* s, const int* chk_dev, const double* alpha_dev);
 int system_enqueue_c_d(mg_system* s);
 // builds the active-pair sublist from the last force_calc's pair values and
 // makes c_d_calc / calc_g walk it (on), or walk the full list again (off);
