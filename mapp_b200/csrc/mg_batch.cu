@@ -548,6 +548,21 @@ struct GatherDst {
     int natms_total;
 };
 
+// one cell's results side by side for one copy to the host: its state, positions
+// and alpha as rows of x_dim, forces
+__global__ void k_cell_result(Dev d, int base, int nat, const CellState* __restrict__ state, CellState* __restrict__ so,
+                              double* __restrict__ x, double* __restrict__ f)
+{
+    dep_sync();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, xd = d.x_dim;
+    if (k == 0) *so = *state;
+    if (k >= nat * xd) return;
+    const int i = base + k / xd, q = k % xd;
+    const double* p = reinterpret_cast<const double*>(d.pos + i);
+    x[k] = q < 3 ? p[q] : d.alpha[(size_t)i * d.nt + q - 3];
+    f[k] = d.f[(size_t)base * xd + k];
+}
+
 __global__ void k_gather_cell(Dev s, GatherDst D, int cell, int obase, int gbase, long long pbase)
 {
     dep_sync();
@@ -781,6 +796,9 @@ struct mg_batch {
     DArr<double4> pos, pos0;
     DArr<double> alpha, c, shift, f, E, dE, pr, partial, cell_E, vec, probe_out;
     DArr<float> prf;
+    DArr<unsigned char> res;  // one cell's results on their way to the host
+    unsigned char* res_host = nullptr;
+    size_t res_host_cap = 0;
     DArr<int4> icut;       // the precision form's in-cut pair list (two int4 per pair)
     DArr<float4> srec;     // and its per-site FP32 records
     DArr<float> dE32, facc;
@@ -796,6 +814,7 @@ struct mg_batch {
     DArr<int> gerr;           // whole-GPU step: a barrier wait timed out
     // launch shapes
     int bps1 = 0, bps2 = 0, lbt = 256, lcs = 1;  // pass grids, L-BFGS threads per CTA and CTAs per cell
+    bool built_in = true;  // neither tuned nor set by the caller
     bool tuned = false, from_cache = false;
     double tune_ms = 0, build_ms = 0;
     // graph
@@ -1202,6 +1221,19 @@ int autotune(mg_batch* b)
     return MG_OK;
 }
 
+// Built-in shape of the L-BFGS step: 1024 threads, and a cluster of up to 4 CTAs
+// per cell while all of them fit the SMs at once -- a step is 2m + 4 reductions
+// over a cell's vectors, one after the other, so a small batch on 256 threads a
+// cell left most of the GPU idle.  Relaxation of 32 cells of 500-4000 sites, 15
+// iterations: 256 x 1 8.96 ms, 1024 x 1 6.57, 1024 x 2 6.22, 1024 x 4 5.92, 1024 x
+// 8 7.05; 200 cells of 500-2000: 256 x 1 21.7 ms, 1024 x 1 20.6, 1024 x 2 21.5.
+void built_in_step(mg_batch* b)
+{
+    b->lbt = 1024;
+    b->lcs = 1;
+    while (b->lcs < 4 && 2 * b->lcs * (int)b->cells.size() <= num_sms()) b->lcs *= 2;
+}
+
 int check_batch(mg_batch* b)
 {
     if (!b) return bfail(MG_ERR_ARG, "null mg_batch");
@@ -1250,6 +1282,8 @@ int mg_batch_destroy(mg_batch* b)
     b->dE.release();
     b->pr.release();
     b->prf.release();
+    b->res.release();
+    if (b->res_host) cudaFreeHost(b->res_host);
     b->icut.release();
     b->srec.release();
     b->dE32.release();
@@ -1340,8 +1374,7 @@ int mg_batch_set_tuning(mg_batch* b, int autotune_on, const char* cache_path)
     b->tuned = false;
     if (!autotune_on) {
         b->bps1 = b->bps2 = 0;
-        b->lbt = 256;
-        b->lcs = 1;
+        b->built_in = true;
     }
     destroy_graph(b);
     return MG_OK;
@@ -1361,6 +1394,7 @@ int mg_batch_set_launch(mg_batch* b, int bps1, int bps2, int lbfgs_threads, int 
     if (lbfgs_cluster == MG_LAUNCH_WHOLE_GPU) lbfgs_cluster = 0;
     b->autotune = 0;
     b->tuned = false;
+    b->built_in = false;
     b->bps1 = bps1;
     b->bps2 = bps2;
     b->lbt = lbfgs_threads;
@@ -1411,7 +1445,8 @@ int mg_batch_relax(mg_batch* b, mg_batch_stats* stats)
     if (b->autotune && !b->tuned) {
         BCHK(autotune(b));
         b->tuned = true;
-    }
+    } else if (!b->autotune && b->built_in)
+        built_in_step(b);
     b->bd.tune_bps = b->bps1;
     b->bd.tune_bps2 = b->bps2;
     BCHK(capture_graph(b));
@@ -1499,23 +1534,29 @@ int mg_batch_cell_result(mg_batch* b, int cell, double* x, double* f, mg_cell_re
     BCHK(check_batch(b));
     if (!b->built || !b->state.p) return bfail(MG_ERR_STATE, "mg_batch_relax first");
     if (cell < 0 || cell >= (int)b->cells.size()) return bfail(MG_ERR_ARG, "cell %d out of range", cell);
-    const int nat = b->h_nat[cell], base = b->h_base[cell], xd = b->xd, nt = b->nt;
-    if (x) {
-        std::vector<double4> hp(nat);
-        std::vector<double> ha((size_t)nat * nt);
-        BCU(cudaMemcpy(hp.data(), b->pos.p + base, nat * sizeof(double4), cudaMemcpyDeviceToHost));
-        BCU(cudaMemcpy(ha.data(), b->alpha.p + (size_t)base * nt, ha.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        for (int k = 0; k < nat; k++) {
-            x[(size_t)k * xd + 0] = hp[k].x;
-            x[(size_t)k * xd + 1] = hp[k].y;
-            x[(size_t)k * xd + 2] = hp[k].z;
-            for (int t = 0; t < nt; t++) x[(size_t)k * xd + 3 + t] = ha[(size_t)k * nt + t];
-        }
+    const int nat = b->h_nat[cell], base = b->h_base[cell], xd = b->xd;
+    // state, x and f gathered into one block, read with one copy
+    const size_t nv = (size_t)nat * xd, bytes = sizeof(CellState) + 2 * nv * sizeof(double);
+    BCHK(b->res.exact(bytes));
+    if (bytes > b->res_host_cap) {
+        if (b->res_host) cudaFreeHost(b->res_host);
+        b->res_host = nullptr;
+        b->res_host_cap = 0;
+        BCU(cudaMallocHost((void**)&b->res_host, bytes));
+        b->res_host_cap = bytes;
     }
-    if (f) BCU(cudaMemcpy(f, b->f.p + (size_t)base * xd, (size_t)nat * xd * sizeof(double), cudaMemcpyDeviceToHost));
+    double* xv = reinterpret_cast<double*>(b->res.p + sizeof(CellState));
+    launch_dep(k_cell_result, (unsigned)div_up((long long)nv, 256), 256, 0, b->st, b->bd, base, nat,
+               (const CellState*)(b->state.p + cell), reinterpret_cast<CellState*>(b->res.p), xv, xv + nv);
+    BCU(cudaGetLastError());
+    BCU(cudaMemcpyAsync(b->res_host, b->res.p, bytes, cudaMemcpyDeviceToHost, b->st));
+    BCU(cudaStreamSynchronize(b->st));
+    const double* hv = reinterpret_cast<const double*>(b->res_host + sizeof(CellState));
+    if (x) memcpy(x, hv, nv * sizeof(double));
+    if (f) memcpy(f, hv + nv, nv * sizeof(double));
     if (r) {
         CellState s;
-        BCU(cudaMemcpy(&s, b->state.p + cell, sizeof(CellState), cudaMemcpyDeviceToHost));
+        memcpy(&s, b->res_host, sizeof(CellState));
         r->energy = s.E_curr;
         r->max_f = s.max_f;
         r->t_ms = s.t_done * 1e-6;
