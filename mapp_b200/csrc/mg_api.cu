@@ -280,6 +280,8 @@ struct mg_system {
     bool mlp_ready = false;
     float* mlp_loss = nullptr;
     int mlp_loss_n = 0;
+    float *mlp_x = nullptr, *mlp_y = nullptr;  // the training set
+    size_t mlp_set_cap = 0;
     unsigned long long mlp_calls = 0;
     bool skin_pending = false;  // update_x's skin test not yet read (status[7])
     // the value update_x's skin test writes to status[7] when some site moved
@@ -1147,7 +1149,7 @@ int mg_destroy(mg_system* s)
                     s->scan_tmp, s->stage, s->red_out, s->d_rhoT, s->d_phiT, s->d_FT, s->gctl, s->gtiles, s->rb_out};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    void* mptrs[] = {s->mlp.par, s->mlp.wbf, s->mlp.m, s->mlp.v, s->mlp.gpart, s->mlp.audit, s->mlp_loss,
+    void* mptrs[] = {s->mlp.par, s->mlp.wbf, s->mlp.m, s->mlp.v, s->mlp.gpart, s->mlp.audit, s->mlp_loss, s->mlp_x, s->mlp_y,
                      s->mlp.row_in, s->mlp.row_id, s->mlp.row_r, s->mlp.row_n, s->mlp.audit_rows};
     for (void* p : mptrs)
         if (p) cudaFree(p);
@@ -1861,15 +1863,17 @@ int mg_mlp_init(mg_system* s, double r_lo, double r_hi, double w_lo, double w_hi
     if (!s->d_rhoT) CHK(upload_tables(s));
     int np = mlp_nparam(), npart = mlp_npart();
     MlpState& M = s->mlp;
-    CHK(dalloc(&M.par, np));
-    CHK(dalloc((unsigned short**)&M.wbf, np));
-    CHK(dalloc(&M.m, np));
-    CHK(dalloc(&M.v, np));
-    CHK(dalloc(&M.gpart, (size_t)npart * 4096));  // up to 4096 tiles of 64 rows per step
-    CHK(dalloc(&M.audit, 16));
+    // (allocated once: the sizes are fixed, and the partials are 160 MB)
+    if (!M.par) CHK(dalloc(&M.par, np));
+    if (!M.wbf) CHK(dalloc((unsigned short**)&M.wbf, np));
+    if (!M.m) CHK(dalloc(&M.m, np));
+    if (!M.v) CHK(dalloc(&M.v, np));
+    if (!M.gpart) CHK(dalloc(&M.gpart, (size_t)npart * 4096));  // up to 4096 tiles of 64 rows per step
+    if (!M.audit) CHK(dalloc(&M.audit, 16));
     if (!M.row_n) CHK(dalloc(&M.row_n, 4));
-    CU(cudaMemset(M.m, 0, np * sizeof(float)));
-    CU(cudaMemset(M.v, 0, np * sizeof(float)));
+    CU(cudaMemsetAsync(M.m, 0, np * sizeof(float), s->st));
+    CU(cudaMemsetAsync(M.v, 0, np * sizeof(float), s->st));
+    CU(cudaStreamSynchronize(s->st));
     M.box.r_lo = (float)r_lo;
     M.box.r_hi = (float)r_hi;
     M.box.w_lo = (float)w_lo;
@@ -1941,9 +1945,13 @@ int mg_mlp_train(mg_system* s, long long nsamples, int steps, int batch, double 
         return fail(MG_ERR_ARG, "need nsamples >= 64, steps >= 1, batch a multiple of 64 up to 262144");
     if (nsamples > (1LL << 31) - 1) return fail(MG_ERR_ARG, "too many samples");
     int n = (int)nsamples;
-    float *X = nullptr, *Y = nullptr;
-    CHK(dalloc(&X, (size_t)n * 4));
-    CHK(dalloc(&Y, (size_t)n * 6));
+    if ((size_t)n > s->mlp_set_cap) {
+        s->mlp_set_cap = 0;
+        CHK(dalloc(&s->mlp_x, (size_t)n * 4));
+        CHK(dalloc(&s->mlp_y, (size_t)n * 6));
+        s->mlp_set_cap = n;
+    }
+    float *X = s->mlp_x, *Y = s->mlp_y;
     fill_dev_scalars(s);
     CU(launch_mlp_labels(s->d, s->mlp.box, seed, n, X, Y, s->st));
     // output standardisation from the labels
@@ -1973,8 +1981,6 @@ int mg_mlp_train(mg_system* s, long long nsamples, int steps, int batch, double 
     float last = 0.f;
     CU(cudaMemcpyAsync(&last, s->mlp_loss + steps - 1, sizeof(float), cudaMemcpyDeviceToHost, s->st));
     CU(cudaStreamSynchronize(s->st));
-    cudaFree(X);
-    cudaFree(Y);
     if (final_loss) *final_loss = last;
     return MG_OK;
 }

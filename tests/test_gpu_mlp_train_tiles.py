@@ -43,11 +43,18 @@ def test_gradient_blocks(tmp_path, n, kind):
         assert a @ b >= 0.9999 * np.linalg.norm(a) * np.linalg.norm(b), name
 
 
-def test_training_is_reproducible(tmp_path):
+@pytest.mark.parametrize("steps", [60, 200])
+def test_training_is_reproducible(tmp_path, steps):
+    """Also on the legacy default stream and with a larger sample set before."""
     s = _system(tmp_path)
     runs = []
-    for _ in range(2):
+    for k in range(3):
+        if k == 2:
+            s.mlp_train(nsamples=20000, steps=2, batch=64, seed=1)
+            s.set_stream(0)
         s.mlp_init(*BOX, seed=9)
-        s.mlp_train(nsamples=5000, steps=60, batch=640, seed=3)
-        runs.append(s.mlp_state()[0])
-    assert np.array_equal(runs[0].view(np.uint32), runs[1].view(np.uint32))
+        s.mlp_train(nsamples=5000, steps=steps, batch=640, seed=3)
+        runs.append((s.mlp_state()[0], s.mlp_loss_history(steps)))
+    for p, h in runs[1:]:
+        assert np.array_equal(runs[0][0].view(np.uint32), p.view(np.uint32))
+        assert np.array_equal(runs[0][1], h)
