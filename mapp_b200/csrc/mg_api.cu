@@ -1589,7 +1589,11 @@ int mg_ff_force_calc(mg_system* s, int st_clc, double* f, double* en_st)
 int mg_ff_energy_calc(mg_system* s, double* energy)
 {
     MG_NVTX("mg_ff_energy_calc");
-    CHK(check_sys(s));
+    CHK(check_sys_nores(s));
+    // as force_calc: with update_x's skin test pending the energy is computed on
+    // the current list and the test read with the result (a line search calls
+    // update_x and energy_calc in turn, and would wait twice a step otherwise)
+    const bool speculative = s->skin_pending;
     if (!s->initialized) return fail(MG_ERR_STATE, "energy_calc before init");
     if (s->natms == 0) {
         if (energy) *energy = 0.0;
@@ -1607,8 +1611,16 @@ int mg_ff_energy_calc(mg_system* s, double* energy)
     }
     CU(launch_reduce_partials(d, rows, 1, s->red_out, s->st));
     CHK(timed_end(s));
-    CU(cudaMemcpyAsync(s->hp->tot, s->red_out, sizeof(double), cudaMemcpyDeviceToHost, s->st));
+    CU(cudaMemcpyAsync(s->hp, s->red_out, 8 * sizeof(double) + 8 * sizeof(int), cudaMemcpyDeviceToHost, s->st));
     CU(cudaStreamSynchronize(s->st));
+    if (speculative) {
+        s->skin_pending = false;
+        if (s->hp->status[7] == s->skin_gen) {
+            CU(launch_x2s(d, s->st));
+            CHK(rebuild(s));
+            return mg_ff_energy_calc(s, energy);
+        }
+    }
     CHK(timed_read(s, &s->t_energy));
     if (energy) *energy = s->hp->tot[0];
     return MG_OK;
