@@ -236,6 +236,9 @@ struct mg_system {
     int cap_bins = 0;
     void* scan_tmp = nullptr;
     size_t scan_tmp_bytes = 0;
+    char* ws = nullptr;  // workspace of the device-resident runs (system_workspace)
+    void* ws_host = nullptr;
+    size_t ws_cap = 0, ws_host_cap = 0;
     double* stage = nullptr;  // device staging for host arrays
     size_t stage_cap = 0;
     size_t act_cap = 0;   // capacity of the active-pair sublist (entries)
@@ -1146,7 +1149,7 @@ int mg_destroy(mg_system* s)
     void* ptrs[] = {d.prf, s->d_pkT, s->d_pk64, s->d_pkS, d.icut, d.icut_n, d.srec, d.dE32, d.facc, d.poff, d.pair_i, d.pair_j, d.pos, d.sfr, d.pos0, d.alpha, d.c, d.type, d.root, d.gchain, d.bin, d.cell_start,
                     d.cell_count, d.cell_pos, d.nbr, d.nnb, d.crdl, d.ncrd, d.crd, d.f, d.rho, d.E,
                     d.dE, d.ddE, d.n, d.s, d.t, d.v, d.c_d, d.a_in, d.g, d.pr, d.partial, d.act_pj, d.act_pv, d.act_off, d.nact,
-                    s->scan_tmp, s->stage, s->red_out, s->d_rhoT, s->d_phiT, s->d_FT, s->gctl, s->gtiles, s->rb_out};
+                    s->scan_tmp, s->stage, s->red_out, s->d_rhoT, s->d_phiT, s->d_FT, s->gctl, s->gtiles, s->rb_out, s->ws};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* mptrs[] = {s->mlp.par, s->mlp.wbf, s->mlp.m, s->mlp.v, s->mlp.gpart, s->mlp.audit, s->mlp_loss, s->mlp_x, s->mlp_y,
@@ -1164,6 +1167,7 @@ int mg_destroy(mg_system* s)
     if (s->ev_join) cudaEventDestroy(s->ev_join);
     if (s->side) cudaStreamDestroy(s->side);
     if (s->hp) cudaFreeHost(s->hp);
+    if (s->ws_host) cudaFreeHost(s->ws_host);
     delete s;
     return MG_OK;
 }
@@ -2113,6 +2117,24 @@ int mg::system_enqueue_force(mg_system* s, int st_clc, int zero, int* rows)
         CU(launch_zero(d.f, (size_t)s->natms * s->x_dim, d.rho, (size_t)s->natms, s->st));
     }
     CU(s->style == STYLE_EAM ? launch_eam_force(d, st_clc, rows, s->st) : launch_fs_force(d, st_clc, rows, s->st));
+    return MG_OK;
+}
+int mg::system_workspace(mg_system* s, size_t dev_bytes, size_t host_bytes, void** dev, void** host)
+{
+    if (dev_bytes > s->ws_cap) {
+        s->ws_cap = 0;
+        CHK(dalloc(&s->ws, dev_bytes));
+        s->ws_cap = dev_bytes;
+    }
+    if (host_bytes > s->ws_host_cap) {
+        if (s->ws_host) cudaFreeHost(s->ws_host);
+        s->ws_host = nullptr;
+        s->ws_host_cap = 0;
+        CU(cudaMallocHost(&s->ws_host, host_bytes));
+        s->ws_host_cap = host_bytes;
+    }
+    *dev = s->ws;
+    *host = s->ws_host;
     return MG_OK;
 }
 double* mg::system_red_out(mg_system* s) { return s->red_out; }

@@ -586,9 +586,21 @@ struct Clock {
     {
         if (ls_exec) cudaGraphExecDestroy(ls_exec);
         if (ls_graph) cudaGraphDestroy(ls_graph);
-        cudaFree(S_dev);
-        cudaFree(block);
-        if (hout) cudaFreeHost(hout);
+    }
+
+    // the vectors and scalars (n doubles), the solve's device state and the
+    // page-locked block: a workspace the system keeps, since freeing and
+    // allocating it in every run synchronises and at times takes milliseconds
+    int workspace(size_t n)
+    {
+        constexpr size_t head = (sizeof(SolveDev) + 255) / 256 * 256;
+        void *dev = nullptr, *host = nullptr;
+        KCHK(system_workspace(s, head + n * sizeof(double), sizeof(HostOut), &dev, &host));
+        S_dev = reinterpret_cast<SolveDev*>(dev);
+        block = reinterpret_cast<double*>(reinterpret_cast<char*>(dev) + head);
+        hout = reinterpret_cast<HostOut*>(host);
+        host_sc = hout->sc;
+        return MG_OK;
     }
 
     int grid() const { return V.nblocks; }
@@ -611,9 +623,6 @@ struct Clock {
     // graph: k_bs_init, then WHILE (condition set by k_bs_init and bs_fin)
     int build_ls_graph()
     {
-        KCU(cudaMalloc(&S_dev, sizeof(SolveDev)));
-        KCU(cudaMallocHost((void**)&hout, sizeof(HostOut)));
-        host_sc = hout->sc;
         KCU(cudaGraphCreate(&ls_graph, 0));
         cudaGraphConditionalHandle h;
         KCU(cudaGraphConditionalHandleCreate(&h, ls_graph, 0, cudaGraphCondAssignDefault));
@@ -913,15 +922,9 @@ struct ActivePairs {
 
 int clock_force_init(mg_system* s)
 {
-    int style = -1, nt = 0, x_dim = 0, form = 0;
-    system_shape(s, &style, &nt, &x_dim, &form, nullptr);
-    const int natms = system_natms(s);
     KCHK(mg_ff_create_2nd_neigh_lst(s));
-    double* fdev = nullptr;
-    KCU(cudaMalloc(&fdev, ((size_t)natms * x_dim + 1) * sizeof(double)));
     double en[7];
-    int rc = mg_ff_force_calc(s, 1, fdev, en);
-    cudaFree(fdev);
+    const int rc = mg_ff_force_calc(s, 1, nullptr, en);
     if (rc != MG_OK) return rc;
     return system_set_active_pairs(s, true);
 }
@@ -959,7 +962,7 @@ extern "C" int mg_clock_adams(mg_system* s, int order, int nsteps, double delta_
     const int nblocks = div_up(n, kCkBlock);
     size_t vec = ((size_t)n + 31) / 32 * 32;
     size_t total = vec * (3 + m) + (size_t)nblocks * 8 + SC_COUNT + 8;
-    KCU(cudaMalloc(&ck.block, total * sizeof(double)));
+    KCHK(ck.workspace(total));
     Dev& d = system_dev(s);
     ck.V.c = d.c;
     ck.V.c_d = d.c_d;
@@ -1056,7 +1059,7 @@ extern "C" int mg_clock_bdf(mg_system* s, int nsteps, const mg_bdf_opts* opts, d
     const int mo = o.max_order, nblocks = div_up(n, kCkBlock);
     const size_t vec = ((size_t)n + 31) / 32 * 32;
     const size_t total = vec * (6 + mo) + (size_t)nblocks * 8 + SC_COUNT + 8;
-    KCU(cudaMalloc(&ck.block, total * sizeof(double)));
+    KCHK(ck.workspace(total));
     Dev& d = system_dev(s);
     ck.V.c = d.c;
     ck.V.c_d = d.c_d;

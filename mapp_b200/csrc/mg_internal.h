@@ -350,6 +350,9 @@ int system_check_ready(mg_system* s);
 void system_masses(mg_system* s, double* out);
 // x2s of the owned atoms, then the ghost / bin / list rebuild (Atoms::update_0's rebuild branch)
 int system_rebuild(mg_system* s);
+// a device and a page-locked block of at least these sizes, kept by the system
+// for its device-resident runs (one at a time; contents undefined)
+int system_workspace(mg_system* s, size_t dev_bytes, size_t host_bytes, void** dev, void** host);
 // enqueue force_calc's device work only (zero f and rho unless the caller has,
 // the EAM / FS passes); capturable
 int system_enqueue_force(mg_system* s, int st_clc, int zero, int* rows);
