@@ -783,7 +783,7 @@ cudaError_t dmd32_tail_nt(const Dev& d, int st_clc, int row0, int* nb, cudaStrea
     int g1 = persistent_grid(d.npairs, d.tune_bps2 > 0 ? d.tune_bps2 : MG_DMD32_MINB), g2 = div_up(d.natms, kFFBlock);
     launch_dep(k_dmd32_embed<NT>, g2, kFFBlock, 0, st, d, row0);
     if (evs) cudaEventRecord(evs[2], st);
-    launch_dep(k_dmd32_pass2<NT>, g1, kFFBlock, 0, st, d, st_clc, row0 + g2);
+    launch_full(k_dmd32_pass2<NT>, g1, kFFBlock, 0, st, d, st_clc, row0 + g2);
     if (evs) cudaEventRecord(evs[3], st);
     *nb = g1 + g2;
     return cudaGetLastError();

@@ -749,19 +749,19 @@ cudaError_t mlp_force_nt(const Dev& d, const MlpState& S, unsigned long long aud
     cudaError_t e = cudaMemsetAsync(S.row_n, 0, 4 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     if (evs) cudaEventRecord(evs[0], st);
-    launch_dep(k_mlp_rows<NT>, std::max(g0, 1), kFFBlock, 0, st, d, S, audit_seed);
+    launch_full(k_mlp_rows<NT>, std::max(g0, 1), kFFBlock, 0, st, d, S, audit_seed);
     const size_t smF = (size_t)(NT * NT + NT * (NT + 1) / 2) * d.nrS * sizeof(float4);
     if (smF > 48 * 1024) {
         e = cudaFuncSetAttribute(nq3 ? k_mlp_fallback<NT, 3> : k_mlp_fallback<NT, 0>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smF);
         if (e != cudaSuccess) return e;
     }
-    if (nq3) launch_dep(k_mlp_fallback<NT, 3>, num_sms() * 4, kFFBlock, smF, st, d, S);
-    else launch_dep(k_mlp_fallback<NT, 0>, num_sms() * 4, kFFBlock, smF, st, d, S);
-    launch_dep(k_mlp_tc<NT, ACT>, g1, kTcThreads, sm, st, d, S);
-    if (d.nq == 3) launch_dep(k_mlp_audit<NT, 3>, num_sms(), kFFBlock, 0, st, d, S);
-    else launch_dep(k_mlp_audit<NT, 0>, num_sms(), kFFBlock, 0, st, d, S);
-    launch_dep(k_mlp_densities<NT>, gd, kFFBlock, 0, st, d, 0);
+    if (nq3) launch_full(k_mlp_fallback<NT, 3>, num_sms() * 4, kFFBlock, smF, st, d, S);
+    else launch_full(k_mlp_fallback<NT, 0>, num_sms() * 4, kFFBlock, smF, st, d, S);
+    launch_full(k_mlp_tc<NT, ACT>, g1, kTcThreads, sm, st, d, S);
+    if (d.nq == 3) launch_full(k_mlp_audit<NT, 3>, num_sms(), kFFBlock, 0, st, d, S);
+    else launch_full(k_mlp_audit<NT, 0>, num_sms(), kFFBlock, 0, st, d, S);
+    launch_full(k_mlp_densities<NT>, gd, kFFBlock, 0, st, d, 0);
     if (evs) cudaEventRecord(evs[1], st);
     int rows = 0;
     e = launch_dmd_force_f32_after_pass1(d, st_clc, gd, &rows, st, evs);
