@@ -1546,7 +1546,13 @@ int mg_batch_cell_result(mg_batch* b, int cell, double* x, double* f, mg_cell_re
         b->res_host_cap = bytes;
     }
     double* xv = reinterpret_cast<double*>(b->res.p + sizeof(CellState));
-    launch_dep(k_cell_result, (unsigned)div_up((long long)nv, 256), 256, 0, b->st, b->bd, base, nat,
+    // the arrays as they are now: a relaxation that failed in its list build may
+    // have moved them after bd was filled
+    Dev d = b->bd;
+    d.pos = b->pos.p;
+    d.alpha = b->alpha.p;
+    d.f = b->f.p;
+    launch_dep(k_cell_result, (unsigned)div_up((long long)nv, 256), 256, 0, b->st, d, base, nat,
                (const CellState*)(b->state.p + cell), reinterpret_cast<CellState*>(b->res.p), xv, xv + nv);
     BCU(cudaGetLastError());
     BCU(cudaMemcpyAsync(b->res_host, b->res.p, bytes, cudaMemcpyDeviceToHost, b->st));
