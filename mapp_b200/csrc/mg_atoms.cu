@@ -33,7 +33,7 @@ __device__ __forceinline__ void set3(double4& p, int k, double v)
     else p.z = v;
 }
 
-__global__ void k_split_x(Dev d, const double* __restrict__ x, int frac)
+__global__ void k_split_x(Dev d, const double* x, int frac)
 {
     dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -97,7 +97,7 @@ __global__ void k_x2s(Dev d)
 constexpr int kGhostTile = 2 * kBlock;
 constexpr unsigned kTileAgg = 1u << 30, kTilePrefix = 1u << 31, kTileVal = (1u << 30) - 1;
 
-__global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* __restrict__ c, GhostCtl* __restrict__ nx,
+__global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* c, GhostCtl* __restrict__ nx,
                                                        unsigned* __restrict__ tiles, unsigned* __restrict__ tiles_next,
                                                        int* __restrict__ ticket, int* __restrict__ ticket_next, int cap,
                                                        int dim, int dir, int next_mode)
@@ -387,9 +387,8 @@ __global__ void __launch_bounds__(kClusterThreads) k_ghost_cluster(Dev d, GhostC
 // control, the status words and the total (the last output).
 constexpr int kScanSmall = 65536;
 
-__global__ void __launch_bounds__(1024) k_scan_small(const int* __restrict__ in, int* __restrict__ out, int n,
-                                                     const GhostCtl* __restrict__ gc, const int* __restrict__ status,
-                                                     RebuildOut* __restrict__ rb)
+__global__ void __launch_bounds__(1024) k_scan_small(const int* in, int* out, int n,
+                                                     const GhostCtl* gc, const int* status, RebuildOut* rb)
 {
     dep_sync();
     __shared__ int s_w[32];
@@ -462,7 +461,7 @@ __device__ __forceinline__ int nall_of(const Dev& d, const GhostCtl* gc, int cap
 
 // Neighbor::s2bin for every atom, then Atoms::s2x (owned + ghost), counting
 // atoms per bin.
-__global__ void k_bin_s2x(Dev d, const GhostCtl* __restrict__ gc, int cap)
+__global__ void k_bin_s2x(Dev d, const GhostCtl* gc, int cap)
 {
     dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -492,7 +491,7 @@ __device__ __forceinline__ double pack_idx(int idx, int type)
 __device__ __forceinline__ int unpack_idx(double w) { return (int)(__double_as_longlong(w) & 0xffffffffll); }
 __device__ __forceinline__ int unpack_type(double w) { return (int)(__double_as_longlong(w) >> 32); }
 
-__global__ void k_cell_fill(Dev d, int* __restrict__ cursor, const GhostCtl* __restrict__ gc, int cap)
+__global__ void k_cell_fill(Dev d, int* __restrict__ cursor, const GhostCtl* gc, int cap)
 {
     dep_sync();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -594,7 +593,7 @@ __global__ void k_store_x0(Dev d)
 // straight from the caller's x (roots are owned sites), so no second launch has
 // to wait for the owned copy.  A site past the skin writes `gen`, which the
 // caller makes new for every call, to *flag, so the word needs no reset.
-__global__ void k_update_x(Dev d, const double* __restrict__ x, double sq_skin, int* __restrict__ flag, int gen)
+__global__ void k_update_x(Dev d, const double* x, double sq_skin, int* __restrict__ flag, int gen)
 {
     dep_sync();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -651,7 +650,7 @@ __global__ void k_merge_x(Dev d, double* __restrict__ x, int first, int count)
 // Deterministic final reduction of per-block partial sums: one block of 1024
 // threads; each thread sums its strided rows for all columns at once (rows are
 // 64-byte records), then a warp-shuffle and shared-memory tree per column.
-__global__ void __launch_bounds__(1024) k_reduce_partials(const double* __restrict__ partial, int nblocks, int nvals,
+__global__ void __launch_bounds__(1024) k_reduce_partials(const double* partial, int nblocks, int nvals,
                                                          double* __restrict__ out)
 {
     dep_sync();

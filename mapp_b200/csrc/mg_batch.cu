@@ -518,7 +518,7 @@ __global__ void k_zero_active(Dev d, int ncells)
 }
 
 // ghosts of running cells from their owners (position + image shift, alpha)
-__global__ void k_refresh_ghosts(Dev d, const double* __restrict__ shift, const unsigned char* __restrict__ active)
+__global__ void k_refresh_ghosts(Dev d, const double* shift, const unsigned char* active)
 {
     dep_sync();
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -550,7 +550,7 @@ struct GatherDst {
 
 // one cell's results side by side for one copy to the host: its state, positions
 // and alpha as rows of x_dim, forces
-__global__ void k_cell_result(Dev d, int base, int nat, const CellState* __restrict__ state, CellState* __restrict__ so,
+__global__ void k_cell_result(Dev d, int base, int nat, const CellState* state, CellState* __restrict__ so,
                               double* __restrict__ x, double* __restrict__ f)
 {
     dep_sync();

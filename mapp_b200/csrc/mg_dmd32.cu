@@ -115,11 +115,13 @@ __device__ __forceinline__ float seg_sumf(float v, const Seg& s)
     return v;
 }
 
-// a site position as one 32-byte read-only load
+// a site position as one 32-byte load (volatile: it stays behind dep_sync)
 __device__ __forceinline__ double4 pos_ld(const Dev& d, int i)
 {
     double4 r;
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(d.pos + i));
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w)
+                 : "l"(d.pos + i));
     return r;
 }
 
@@ -128,13 +130,13 @@ template <int NT>
 __device__ __forceinline__ void load_rec(const Dev& d, int j, float (&al)[NT], float (&cc)[NT])
 {
     float v[8];
-    const float4 r0 = __ldg(d.srec + (size_t)j * kSiteRec);
+    const float4 r0 = d.srec[(size_t)j * kSiteRec];
     v[0] = r0.x;
     v[1] = r0.y;
     v[2] = r0.z;
     v[3] = r0.w;
     if (2 * NT > 4) {
-        const float4 r1 = __ldg(d.srec + (size_t)j * kSiteRec + 1);
+        const float4 r1 = d.srec[(size_t)j * kSiteRec + 1];
         v[4] = r1.x;
         v[5] = r1.y;
         v[6] = r1.z;
@@ -370,7 +372,7 @@ __global__ void MG_FORCE_BOUNDS k_dmd32_force(Dev d, int st_clc, int row0, int W
     float vir[6] = {0, 0, 0, 0, 0, 0};
     for (long long t = (long long)blockIdx.x * kFFWarps + (threadIdx.x >> 5); t < nslot; t += wstride) {
         const long long rg = t / K;
-        if (t - rg * K >= (long long)__ldg(d.icut_n + rg)) continue;  // past the region's last batch
+        if (t - rg * K >= (long long)d.icut_n[rg]) continue;  // past the region's last batch
         const int4 e = d.icut[(size_t)t * 64 + lane];
         const int4 ex = d.icut[(size_t)t * 64 + 32 + lane];
         const bool on = e.x >= 0;
@@ -407,8 +409,8 @@ __global__ void MG_FORCE_BOUNDS k_dmd32_force(Dev d, int st_clc, int row0, int W
             const bool own_j = j < d.natms;
             float dEi[NT], dEj[NT];
             if (NT == 2) {
-                const float2 ei = __ldg(reinterpret_cast<const float2*>(d.dE32) + i);
-                const float2 ej = __ldg(reinterpret_cast<const float2*>(d.dE32) + oj);
+                const float2 ei = reinterpret_cast<const float2*>(d.dE32)[i];
+                const float2 ej = reinterpret_cast<const float2*>(d.dE32)[oj];
                 dEi[0] = ei.x;
                 dEi[NT - 1] = ei.y;
                 dEj[0] = ej.x;
@@ -416,8 +418,8 @@ __global__ void MG_FORCE_BOUNDS k_dmd32_force(Dev d, int st_clc, int row0, int W
             } else {
 #pragma unroll
                 for (int a = 0; a < NT; a++) {
-                    dEi[a] = __ldg(d.dE32 + (size_t)i * NT + a);
-                    dEj[a] = __ldg(d.dE32 + (size_t)oj * NT + a);
+                    dEi[a] = d.dE32[(size_t)i * NT + a];
+                    dEj[a] = d.dE32[(size_t)oj * NT + a];
                 }
             }
             const Knot k0 = knot_at(r, k);

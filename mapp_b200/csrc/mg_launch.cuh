@@ -7,6 +7,13 @@
 // while the one before it runs; its blocks wait in dep_sync, its first
 // statement, until everything before it in the stream is complete and visible.
 // Behind a copy or an event it starts as any other launch does.
+//
+// Such a kernel is resident while the one before it still writes its inputs, so
+// it reads what an earlier kernel of the chain writes with plain loads (or from
+// L2, __ldcg): the read-only path (__ldg, ld.global.nc, and a kernel parameter
+// that is const and __restrict__, which the compiler may turn into it) asks for
+// data that does not change while the kernel lives, and is not ordered by the
+// wait.  It is for the potential tables alone.
 #pragma once
 
 #include <cuda_runtime.h>

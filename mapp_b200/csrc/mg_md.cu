@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kMdBlock) k_md_kick_drift(Dev d, NhConst C, Nh
 // x_0, and force_calc's zeroing of f and rho.  The last block sets the while
 // node's condition: go on unless a rebuild is due or the run is over.
 __global__ void __launch_bounds__(kMdBlock) k_md_center(Dev d, NhConst C, NhState* S,
-                                                        const double4* __restrict__ xu,
+                                                        const double4* xu,
                                                         cudaGraphConditionalHandle handle, int set_cond)
 {
     dep_sync();

@@ -296,7 +296,7 @@ __device__ __forceinline__ void warp_gemm8(const __nv_bfloat16* A, int lda, cons
     }
 }
 
-__device__ __forceinline__ void load_w(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int rows, int first, int k)
+__device__ __forceinline__ void load_w(__nv_bfloat16* dst, const __nv_bfloat16* src, int rows, int first, int k)
 {
     // 16-byte piece k - first of a [rows][64] matrix, into rows of pitch HP
     const int e = k - first;
@@ -304,8 +304,7 @@ __device__ __forceinline__ void load_w(__nv_bfloat16* dst, const __nv_bfloat16* 
         *reinterpret_cast<uint4*>(dst + (e >> 3) * HP + (e & 7) * 8) = *reinterpret_cast<const uint4*>(src + e * 8);
 }
 
-__global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpState S, const float* __restrict__ X,
-                                                             const float* __restrict__ Y, int n, int batch,
+__global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpState S, const float* X, const float* Y, int n, int batch,
                                                              unsigned long long seed, int step, int fixed)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -264,7 +264,7 @@ __device__ __forceinline__ void base_f32(const Dev& d, int aa, int bb, float r, 
 
 // B operand of one layer: element (n, k) = W[k][n] of the row-major [K][N]
 // weights (n >= nsrc zero)
-__device__ __forceinline__ void load_b(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ w, int rows, int nsrc,
+__device__ __forceinline__ void load_b(__nv_bfloat16* dst, const __nv_bfloat16* w, int rows, int nsrc,
                                        int K)
 {
     for (int e = threadIdx.x; e < rows * K; e += blockDim.x) {
@@ -559,9 +559,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_tc(Dev d, MlpState S)
     const long long tstride = (long long)gridDim.x * kPipes;
     // this thread's row of the next tile, loaded one tile ahead
     long long rw = t * kTile + row;
-    float4 in = rw < nrows ? __ldg(S.row_in + rw) : make_float4(0.f, 0.f, 0.f, 0.f);
-    int2 id = rw < nrows ? __ldg(S.row_id + rw) : make_int2(-1, 0);
-    float rr = rw < nrows ? __ldg(S.row_r + rw) : 1.0f;
+    float4 in = rw < nrows ? S.row_in[rw] : make_float4(0.f, 0.f, 0.f, 0.f);
+    int2 id = rw < nrows ? S.row_id[rw] : make_int2(-1, 0);
+    float rr = rw < nrows ? S.row_r[rw] : 1.0f;
     for (; t < ntiles; t += tstride) {
         const bool on = rw < nrows;
         const int2 cid = id;
@@ -570,9 +570,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_tc(Dev d, MlpState S)
             make_uint4(pack2f(in.x, in.y), pack2f(in.z, in.w), 0u, 0u);
         rw = (t + tstride) * kTile + row;
         if (rw < nrows) {
-            in = __ldg(S.row_in + rw);
-            id = __ldg(S.row_id + rw);
-            rr = __ldg(S.row_r + rw);
+            in = S.row_in[rw];
+            id = S.row_id[rw];
+            rr = S.row_r[rw];
         }
         if (!mma_step(a0, T.w1, H, 1)) { failed = true; break; }
         epilogue64<ACT>(tlane, T.b1, a1, row);
@@ -689,11 +689,11 @@ __global__ void __launch_bounds__(kFFBlock, 4) k_mlp_densities(Dev d, int row0)
             for (int a = 0; a < NT; a++)
 #pragma unroll
                 for (int b = 0; b < NT; b++) {
-                    const double g0 = (double)__ldg(in + (SL::RHO + b * NT + a) * mp);
+                    const double g0 = (double)in[(SL::RHO + b * NT + a) * mp];
                     Ei[a] += g0 * cj[b];
                     Ej[b] += g0 * ci[a];
                     if (a >= b)
-                        acc[0] += w * (cj[b] * ci[a] + cj[a] * ci[b]) * (double)__ldg(in + (SL::PHI + comp_idx(a, b)) * mp);
+                        acc[0] += w * (cj[b] * ci[a] + cj[a] * ci[b]) * (double)in[(SL::PHI + comp_idx(a, b)) * mp];
                 }
             if (own_j)
 #pragma unroll
