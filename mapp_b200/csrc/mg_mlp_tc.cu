@@ -759,8 +759,13 @@ cudaError_t mlp_force_nt(const Dev& d, const MlpState& S, unsigned long long aud
     if (nq3) launch_full(k_mlp_fallback<NT, 3>, num_sms() * 4, kFFBlock, smF, st, d, S);
     else launch_full(k_mlp_fallback<NT, 0>, num_sms() * 4, kFFBlock, smF, st, d, S);
     launch_full(k_mlp_tc<NT, ACT>, g1, kTcThreads, sm, st, d, S);
-    if (d.nq == 3) launch_full(k_mlp_audit<NT, 3>, num_sms(), kFFBlock, 0, st, d, S);
-    else launch_full(k_mlp_audit<NT, 0>, num_sms(), kFFBlock, 0, st, d, S);
+    // (a plain launch at every size: queued early, the audit's blocks wait on the
+    // SMs for as long as the network's persistent CTAs run, and the call is slower
+    // for it -- 256 sites 163 us either way, 32000 582 us instead of 579, 62500
+    // 973 instead of 962, 500000 6392 instead of 6324)
+    if (d.nq == 3) k_mlp_audit<NT, 3><<<num_sms(), kFFBlock, 0, st>>>(d, S);
+    else k_mlp_audit<NT, 0><<<num_sms(), kFFBlock, 0, st>>>(d, S);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     launch_full(k_mlp_densities<NT>, gd, kFFBlock, 0, st, d, 0);
     if (evs) cudaEventRecord(evs[1], st);
     int rows = 0;

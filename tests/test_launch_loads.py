@@ -69,3 +69,10 @@ def test_read_only_loads_are_the_tables():
     for name, ln in found:
         table = "d.pkS" in ln or (name == "mg_dmd_common.cuh" and ("return __ldg(p);" in ln or '"l"(row)' in ln))
         assert table, (name, ln)
+
+
+def test_the_audit_starts_after_the_network():
+    """Blocks of the learned form's audit that wait beside the persistent network
+    kernel slow it down (1 % of a 500000-site call): a plain launch."""
+    assert "k_mlp_audit" not in _queued()
+    assert "k_mlp_audit<NT, 3><<<" in SRC["mg_mlp_tc.cu"]
