@@ -2036,8 +2036,9 @@ int mg_mlp_grad(mg_system* s, int n, const float* x, const float* y, float* grad
     CHK(dalloc(&Y, (size_t)n * 6));
     CHK(dalloc(&G, (size_t)mlp_nparam()));
     CHK(dalloc(&L, 1));
-    CU(cudaMemcpy(X, x, (size_t)n * 4 * sizeof(float), cudaMemcpyDefault));
-    CU(cudaMemcpy(Y, y, (size_t)n * 6 * sizeof(float), cudaMemcpyDefault));
+    // (on the stream of the step that reads them)
+    CU(cudaMemcpyAsync(X, x, (size_t)n * 4 * sizeof(float), cudaMemcpyDefault, s->st));
+    CU(cudaMemcpyAsync(Y, y, (size_t)n * 6 * sizeof(float), cudaMemcpyDefault, s->st));
     CU(launch_mlp_train_step(s->mlp, X, Y, n, n, 0, 0, 1, 0.0f, 1, G, L, s->st));
     CU(cudaMemcpyAsync(grad, G, mlp_nparam() * sizeof(float), cudaMemcpyDefault, s->st));
     float l = 0;

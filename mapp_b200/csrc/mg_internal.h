@@ -303,6 +303,8 @@ cudaError_t launch_mlp_labels(const Dev& d, const MlpBox& box, unsigned long lon
 // rows of 12 doubles (sums of the six labels, then of their squares), one per block
 int mlp_label_sum_rows(int n);
 cudaError_t launch_mlp_label_sums(const float* Y, int n, double* out, cudaStream_t st);
+// one training step; X and Y filled by work queued on st before the first step
+// (step 0, or fixed) and unchanged until the last one is done
 cudaError_t launch_mlp_train_step(const MlpState& S, const float* X, const float* Y, int n, int batch,
                                   unsigned long long seed, int step, int total, float lr, int fixed, float* grad_out,
                                   float* loss_hist, cudaStream_t st);

@@ -6,6 +6,9 @@
 // BDF clock's iteration at 500 sites (56 us with overlapping starts).  A kernel queued by launch_dep is set up
 // while the one before it runs; its blocks wait in dep_sync, its first
 // statement, until everything before it in the stream is complete and visible.
+// (Two kernels split dep_sync: k_mlp_train reads its rows before the wait and
+// k_mlp_adam lets the next step be set up before it waits; what makes that safe
+// stands at each, and the first step of a run is not queued this way.)
 // Behind a copy or an event it starts as any other launch does.
 //
 // Such a kernel is resident while the one before it still writes its inputs, so
@@ -22,7 +25,7 @@
 
 namespace mg {
 
-// first statement of every kernel that launch_dep queues (a plain launch passes
+// first statement of the kernels that launch_dep queues (a plain launch passes
 // through it): waits for the work before this kernel, then lets the next
 // kernel's blocks be set up
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

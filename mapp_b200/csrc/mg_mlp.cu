@@ -310,7 +310,10 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpState S, const f
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainTile& T = *reinterpret_cast<TrainTile*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    dep_start();  // (before dep_wait: the rows of a tile depend on nothing the previous step writes)
+    // (before dep_wait: a tile's rows depend on nothing a step writes, and until the
+    // wait only this CTA's shared memory is written; the run's first step is launched
+    // plainly, when X and Y are complete)
+    dep_start();
     // 8 threads per row: one takes the inputs, six a target each
     if (tid < kRows * 8) {
         const int r = tid >> 3, part = tid & 7;
@@ -484,8 +487,8 @@ __global__ void __launch_bounds__(kAdamThreads) k_mlp_adam(MlpState S, int nbloc
                            float* __restrict__ loss_hist)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
-    dep_start();
-    if (p > NPARAM) return;
+    dep_start();  // (the next step waits for this kernel before it reads weights or writes partials)
+    if (p > NPARAM) return;  // (every block has threads that go on and wait)
     dep_wait();  // this step's partial gradients
     float g = 0.f;
 #pragma unroll 16
@@ -562,12 +565,18 @@ cudaError_t launch_mlp_train_step(const MlpState& S, const float* X, const float
                                   float* loss_hist, cudaStream_t st)
 {
     constexpr size_t sm = sizeof(TrainTile);
+    const int nb = batch / kRows;
+    cudaError_t e;
     if (step == 0 || fixed) {
-        const cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        // the first step of a run is a plain launch: k_mlp_train reads X and Y before
+        // its wait, so it must not start before the work that fills them is complete;
+        // behind it only steps follow, and those write neither
+        e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-    }
-    int nb = batch / kRows;
-    cudaError_t e = launch_dep(k_mlp_train, nb, kTrainThreads, sm, st, S, X, Y, n, batch, seed, step, fixed);
+        k_mlp_train<<<nb, kTrainThreads, sm, st>>>(S, X, Y, n, batch, seed, step, fixed);
+        e = cudaGetLastError();
+    } else
+        e = launch_dep(k_mlp_train, nb, kTrainThreads, sm, st, S, X, Y, n, batch, seed, step, fixed);
     if (e != cudaSuccess) return e;
     e = launch_dep(k_mlp_adam, div_up(NPARAM + 1, kAdamThreads), kAdamThreads, 0, st, S, nb, step, total, lr, grad_out,
                    loss_hist);

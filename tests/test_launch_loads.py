@@ -76,3 +76,18 @@ def test_the_audit_starts_after_the_network():
     kernel slow it down (1 % of a 500000-site call): a plain launch."""
     assert "k_mlp_audit" not in _queued()
     assert "k_mlp_audit<NT, 3><<<" in SRC["mg_mlp_tc.cu"]
+
+
+def test_the_first_training_step_is_a_plain_launch():
+    """k_mlp_train reads its rows before its wait, so the step that follows the
+    kernels filling them must not be queued early."""
+    t = _strip(SRC["mg_mlp.cu"])
+    body = t[t.index("cudaError_t launch_mlp_train_step("):]
+    first = body[body.index("if (step == 0 || fixed) {"):]
+    first = first[:first.index("}")]
+    assert "k_mlp_train<<<" in first and "launch_dep" not in first
+    assert body.index("launch_dep(k_mlp_train") > body.index("} else")
+    api = _strip(SRC["mg_api.cu"])
+    grad = api[api.index("int mg_mlp_grad("):]
+    grad = grad[:grad.index("launch_mlp_train_step(")]
+    assert grad.count("cudaMemcpyAsync(") == 2 and "cudaMemcpy(" not in grad  # on the step's own stream
