@@ -1951,6 +1951,9 @@ int mg_mlp_state(mg_system* s, float* par_out, const float* par_in, float* scali
     return MG_OK;
 }
 
+// samples of a training set whose buffers stay with the system (40 bytes each: 64 MB)
+static constexpr size_t kMlpSetKept = 1600000;
+
 int mg_mlp_train(mg_system* s, long long nsamples, int steps, int batch, double lr, unsigned long long seed,
                  double* final_loss)
 {
@@ -1961,6 +1964,19 @@ int mg_mlp_train(mg_system* s, long long nsamples, int steps, int batch, double 
         return fail(MG_ERR_ARG, "need nsamples >= 64, steps >= 1, batch a multiple of 64 up to 262144");
     if (nsamples > (1LL << 31) - 1) return fail(MG_ERR_ARG, "too many samples");
     int n = (int)nsamples;
+    // kept for the next run up to kMlpSetKept samples; a larger set is given back on
+    // every way out of this call, as it can take tens of gigabytes
+    struct GiveBack {
+        mg_system* s;
+        ~GiveBack()
+        {
+            if (s->mlp_set_cap && s->mlp_set_cap <= kMlpSetKept) return;
+            cudaFree(s->mlp_x);
+            cudaFree(s->mlp_y);
+            s->mlp_x = s->mlp_y = nullptr;
+            s->mlp_set_cap = 0;
+        }
+    } give_back{s};
     if ((size_t)n > s->mlp_set_cap) {
         s->mlp_set_cap = 0;
         CHK(dalloc(&s->mlp_x, (size_t)n * 4));
