@@ -147,7 +147,8 @@ int mg_get_int_vector(mg_system* s, const char* name, int* out);
    on the system's stream: "list" (always), "force", "energy", "c_d", "calc_g"
    (timing level 1 or 2), and for DMD styles the three force kernels
    "force.pass1", "force.embed", "force.pass2" (level 2); MG_ERR_STATE when the
-   last call of that phase was not timed. */
+   last call of that phase was not timed. "list" is the last build that went
+   through (0 before the first) and waits until it is complete on the stream. */
 int mg_last_time(mg_system* s, const char* phase, double* ms);
 /* Device timing level: 0 no events, 1 (default) one event pair around the
    whole call of force_calc, energy_calc, c_d_calc and calc_g, 2 also an event

@@ -294,8 +294,10 @@ struct mg_system {
     GhostCtl* gctl = nullptr;  // device control of the ghost passes (two, ping-pong)
     unsigned* gtiles = nullptr;  // look-back words of the ghost passes (two halves)
     int gtiles_cap = 0;
-    cudaEvent_t ev_l0 = nullptr, ev_l1 = nullptr;  // around the last list build
-    bool list_timed = false;
+    // around the last list build that went through (pair list_ev; -1: none yet); the
+    // one under way records into the other pair
+    cudaEvent_t ev_list[2][2] = {};
+    int list_ev = -1;
     double t_force = 0, t_energy = 0, t_cd = 0, t_g = 0;
     double t_k[3] = {0, 0, 0};  // DMD force: pass 1, embedding, pass 2
     long long partial_rows = 0;
@@ -561,7 +563,8 @@ int rebuild(mg_system* s)
 {
     Dev& d = s->d;
     cudaStream_t st = s->st;
-    CU(cudaEventRecord(s->ev_l0, st));
+    const int ev = s->list_ev == 0 ? 1 : 0;
+    CU(cudaEventRecord(s->ev_list[ev][0], st));
     int natms = s->natms, nph = 0;
     fill_dev_scalars(s);
     if (!s->gctl) CHK(dalloc(&s->gctl, 2));
@@ -661,8 +664,8 @@ int rebuild(mg_system* s)
     CU(launch_pairs_compact(d, st));
     CU(launch_store_x0(d, st));
     s->crd_built = 0;
-    CU(cudaEventRecord(s->ev_l1, st));  // (read by mg_last_time, so that the host does not wait here)
-    s->list_timed = true;
+    CU(cudaEventRecord(s->ev_list[ev][1], st));  // (read by mg_last_time, so that the host does not wait here)
+    s->list_ev = ev;
     return MG_OK;
 }
 
@@ -1100,8 +1103,8 @@ int mg_create(const char* style, int device, mg_system** out)
     s->own_stream = true;
     cudaEventCreate(&s->ev0);
     cudaEventCreate(&s->ev1);
-    cudaEventCreate(&s->ev_l0);
-    cudaEventCreate(&s->ev_l1);
+    for (auto& pair : s->ev_list)
+        for (cudaEvent_t& e : pair) cudaEventCreate(&e);
     for (int k = 0; k < 4; k++) cudaEventCreate(&s->evk[k]);
     memset(&s->d, 0, sizeof(Dev));
     int r = MG_OK;
@@ -1126,8 +1129,8 @@ int mg_create(const char* style, int device, mg_system** out)
         for (int k = 0; k < 4; k++) cudaEventDestroy(s->evk[k]);
         cudaEventDestroy(s->ev0);
         cudaEventDestroy(s->ev1);
-        cudaEventDestroy(s->ev_l0);
-        cudaEventDestroy(s->ev_l1);
+        for (auto& pair : s->ev_list)
+            for (cudaEvent_t e : pair) cudaEventDestroy(e);
         if (s->ev_fork) cudaEventDestroy(s->ev_fork);
         if (s->ev_join) cudaEventDestroy(s->ev_join);
         if (s->side) cudaStreamDestroy(s->side);
@@ -1158,8 +1161,9 @@ int mg_destroy(mg_system* s)
         if (p) cudaFree(p);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
-    if (s->ev_l0) cudaEventDestroy(s->ev_l0);
-    if (s->ev_l1) cudaEventDestroy(s->ev_l1);
+    for (auto& pair : s->ev_list)
+        for (cudaEvent_t e : pair)
+            if (e) cudaEventDestroy(e);
     for (int k = 0; k < 4; k++)
         if (s->evk[k]) cudaEventDestroy(s->evk[k]);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);
@@ -1809,10 +1813,10 @@ int mg_last_time(mg_system* s, const char* phase, double* ms)
     if (!phase || !ms) return fail(MG_ERR_ARG, "null argument");
     if (!strcmp(phase, "list")) {
         *ms = 0.0;
-        if (s->list_timed) {
+        if (s->list_ev >= 0) {
             float t = 0;
-            CU(cudaEventSynchronize(s->ev_l1));
-            CU(cudaEventElapsedTime(&t, s->ev_l0, s->ev_l1));
+            CU(cudaEventSynchronize(s->ev_list[s->list_ev][1]));
+            CU(cudaEventElapsedTime(&t, s->ev_list[s->list_ev][0], s->ev_list[s->list_ev][1]));
             *ms = t;
         }
     }
