@@ -593,7 +593,7 @@ int rebuild(mg_system* s)
         // holds two arrays of cap_bins), so both are cleared together
         s->cursor = d.cell_count + d.tot_bin + 1;
         const GhostCtl* gfin = s->gctl;
-        if (ghosts_by_cluster(natms)) {
+        if (ghosts_by_cluster(d)) {
             CU(launch_ghost_cluster(d, s->gctl, cap, s->comm_need, d.cell_count, 2 * (d.tot_bin + 1), st));
         } else {
             // the tile words of both halves, then the two tickets: one memset

@@ -230,20 +230,27 @@ __global__ void __launch_bounds__(kBlock) k_ghost_pass(Dev d, const GhostCtl* c,
     }
 }
 
-// The whole of Atoms::ph_setup for systems of up to kClusterSites sites: every
-// pass in one launch of one thread-block cluster, so that a pass costs two
-// cluster barriers instead of a kernel and its look-back chain (six launches, 66
-// us in all at 10000 and 32000 sites; this kernel takes 36 and 54 us, a whole list
-// build 172 -> 102 and 220 -> 149 us).  A pass is a stable
-// compaction: each CTA counts the flagged atoms of its stretch, the counts are
-// exchanged through distributed shared memory, and the stretch is scattered in
-// order.  A dimension that needs one swap pass per direction (every box longer
-// than the cut-off) does both directions at once: the low shell's ghosts, then
-// the high shell's, over the same atoms.  Above kClusterSites the passes want
-// more SMs than a cluster has (42592 sites: 198 us a build by passes, 204 us by
-// the cluster; 108000: 320 and 395).  zero[0..nzero) is the list build's counters,
-// cleared here as well as the status words.
-constexpr int kClusterSites = 40000, kClusterThreads = 1024;
+// The whole of Atoms::ph_setup for builds of up to kClusterSites sites, owned and
+// ghost: every pass in one launch of one thread-block cluster, so that a pass
+// costs two cluster barriers instead of a kernel and its look-back chain.  A pass
+// is a stable compaction: each CTA counts the flagged atoms of its stretch, the
+// counts are exchanged through distributed shared memory, and the stretch is
+// scattered in order.  A dimension that needs one swap pass per direction (every
+// box longer than the cut-off) does both directions at once: the low shell's
+// ghosts, then the high shell's, over the same atoms.  zero[0..nzero) is the list
+// build's counters, cleared here as well as the status words.
+//
+// Where the line lies: the passes read every site made so far, and eight CTAs
+// read them more slowly than the whole GPU does, so the rule looks at all sites
+// (owned ones times 1 + 2 cut-offs per edge) and not at the owned ones: a rod of
+// one cell across has 17 ghosts a site.  A whole list build, by passes and by the
+// cluster, with the sites in all: cubes 117 -> 104 us (14000), 180 -> 150
+// (49000), 234 -> 228 (90000); rods of one cell 153 -> 126 (36000), 168 -> 160
+// (93000), 189 -> 197 (142000); one-cell slabs 182 -> 168 (74000), 222 -> 228
+// (138000).  Three species have more to copy per ghost: cubes 138 -> 132 (28000),
+// 246 -> 253 (90000); slab 195 -> 192 (74000); rods 196 -> 196 (93000).  Fewer CTAs are
+// slower wherever they differ (2000 sites: 104, 92, 91, 85 us with 1, 2, 4, 8).
+constexpr int kClusterSites = 75000, kClusterThreads = 1024, kClusterCtas = 8;
 
 __global__ void __launch_bounds__(kClusterThreads) k_ghost_cluster(Dev d, GhostCtl* __restrict__ out, int cap, int need0,
                                                                    int need1, int need2, int* __restrict__ zero, int nzero)
@@ -722,21 +729,23 @@ cudaError_t launch_ghost_pass(const Dev& d, const GhostCtl* ctl, GhostCtl* next,
     return cudaGetLastError();
 }
 
-bool ghosts_by_cluster(int natms) { return natms <= kClusterSites; }
+bool ghosts_by_cluster(const Dev& d)
+{
+    double sites = d.natms;
+    for (int k = 0; k < 3; k++) sites *= 1.0 + 2.0 * d.cut_ph_s[k];
+    return sites <= kClusterSites;
+}
 
 cudaError_t launch_ghost_cluster(const Dev& d, GhostCtl* out, int cap, const int* need, int* zero, int nzero, cudaStream_t st)
 {
-    // a CTA per 4096 atoms (owned and ghost), 8 at most
-    int cs = 1;
-    while (cs < 8 && cs * 4096 < 2 * d.natms) cs *= 2;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.x = kClusterCtas;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)cs);
+    cfg.gridDim = dim3(kClusterCtas);
     cfg.blockDim = dim3(kClusterThreads);
     cfg.stream = st;
     cfg.attrs = attr;

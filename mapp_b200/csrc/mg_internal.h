@@ -246,9 +246,10 @@ struct RebuildOut {
     int count;  // listed pairs
 };
 cudaError_t launch_ghost_init(const Dev& d, GhostCtl* ctl, cudaStream_t st);
-// every ghost pass in one launch, for systems of up to some ten thousand sites
-// (need: swap passes per dimension); clears the status words and zero[0..nzero)
-bool ghosts_by_cluster(int natms);
+// every ghost pass in one launch, for builds of up to kClusterSites sites,
+// owned and ghost (need: swap passes per dimension); clears the status words and
+// zero[0..nzero)
+bool ghosts_by_cluster(const Dev& d);
 cudaError_t launch_ghost_cluster(const Dev& d, GhostCtl* out, int cap, const int* need, int* zero, int nzero, cudaStream_t st);
 // one ghost pass: tile words and tickets of this pass and of the next
 // (ping-pong halves, ghost_tiles(cap) words each)
