@@ -1221,17 +1221,32 @@ int autotune(mg_batch* b)
     return MG_OK;
 }
 
-// Built-in shape of the L-BFGS step: 1024 threads, and a cluster of up to 4 CTAs
-// per cell while all of them fit the SMs at once -- a step is 2m + 4 reductions
-// over a cell's vectors, one after the other, so a small batch on 256 threads a
-// cell left most of the GPU idle.  Relaxation of 32 cells of 500-4000 sites, 15
-// iterations: 256 x 1 8.96 ms, 1024 x 1 6.57, 1024 x 2 6.22, 1024 x 4 5.92, 1024 x
-// 8 7.05; 200 cells of 500-2000: 256 x 1 21.7 ms, 1024 x 1 20.6, 1024 x 2 21.5.
+// Built-in shape of the minimiser's step, by the largest cell and the number of
+// cells.  A step is 2m + 4 reductions over a cell's vectors, one after the other:
+// small cells want few threads to meet at each, large ones want enough threads for
+// their vectors, and a small batch of large cells leaves most of the GPU idle
+// unless several CTAs (a cluster) share a cell.  us an iteration, L-BFGS with m = 5,
+// FP64 / FP32 passes, at 256 x 1, 512 x 1, 1024 x 1 and 1024 x 4:
+//    32 cells of 32 sites     38 39 45 54            42 40 49 58
+//    32 cells of 256          76 75 83 87            58 61 65 75
+//   148 cells of 256          217 222 222 267        109 110 113 144
+//    32 cells of 500          159 153 159 170        120 114 121 134
+//   512 cells of 500          1584 1588 1642 2107    669 672 726 1191
+//    32 cells of 864          279 261 260 273        197 180 180 193
+//    32 cells of 1372         434 394 385 385        308 266 255 253
+//   200 cells of 1372         2098 2037 2061 2336    902 842 864 1133
+//    32 cells of 4000         1191 1050 992 945      760 615 557 506
+//    74 cells of 4000         2342 2153 2075 2147    1188 1011 931 1005 (1024 x 2: 2044 and 903)
+//   512 cells of 500-8000     9387 9050 8927 9404    4183 3817 3702 4205
+constexpr int kStepSmall = 256, kStepMedium = 1000;  // sites of the largest cell
+
 void built_in_step(mg_batch* b)
 {
-    b->lbt = 1024;
+    const int largest = *std::max_element(b->h_nat.begin(), b->h_nat.end());
     b->lcs = 1;
-    while (b->lcs < 4 && 2 * b->lcs * (int)b->cells.size() <= num_sms()) b->lcs *= 2;
+    b->lbt = largest <= kStepSmall ? 256 : largest <= kStepMedium ? 512 : 1024;
+    if (b->lbt == 1024)
+        while (b->lcs < 4 && 2 * b->lcs * (int)b->cells.size() <= num_sms()) b->lcs *= 2;
 }
 
 int check_batch(mg_batch* b)
