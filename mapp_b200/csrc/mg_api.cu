@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <memory>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -913,35 +914,39 @@ int upload_tables(mg_system* s)
 {
     Dev& d = s->d;
     if (s->style == STYLE_FS || s->tables_uploaded) return MG_OK;
-    CHK(dalloc(&s->d_rhoT, s->rhoT.size()));
-    CHK(dalloc(&s->d_phiT, s->phiT.size()));
     CHK(dalloc(&s->d_FT, s->FT.size()));
-    CU(cudaMemcpy(s->d_rhoT, s->rhoT.data(), s->rhoT.size() * 8, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(s->d_phiT, s->phiT.data(), s->phiT.size() * 8, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(s->d_FT, s->FT.data(), s->FT.size() * 8, cudaMemcpyHostToDevice));
-    d.rhoT = s->d_rhoT;
-    d.phiT = s->d_phiT;
     d.FT = s->d_FT;
+    if (s->dmd) {  // (EAM reads the packed knots below only)
+        CHK(dalloc(&s->d_rhoT, s->rhoT.size()));
+        CHK(dalloc(&s->d_phiT, s->phiT.size()));
+        CU(cudaMemcpy(s->d_rhoT, s->rhoT.data(), s->rhoT.size() * 8, cudaMemcpyHostToDevice));
+        CU(cudaMemcpy(s->d_phiT, s->phiT.data(), s->phiT.size() * 8, cudaMemcpyHostToDevice));
+        d.rhoT = s->d_rhoT;
+        d.phiT = s->d_phiT;
+    }
     {
         // {rho c0..c3, phi c0..c3} per ordered species pair (a, b) and knot,
         // coefficients copied unchanged: the density slot is b*nt+a for the DMD
         // forms, with phi for a >= b, and the one EAM reads for an atom of type a
         // with a neighbour of type b
         const int nt = s->nt, nr = s->nr;
-        std::vector<double> pk64((size_t)nt * nt * nr * 8, 0.0);
+        const size_t np = (size_t)nt * nt * nr * 8;
+        std::unique_ptr<double[]> pk64(new double[np]);
         for (int a = 0; a < nt; a++)
-            for (int b = 0; b < nt; b++)
-                for (int m = 0; m < nr; m++) {
-                    double* dst = pk64.data() + (((size_t)(a * nt + b) * nr + m) * 8);
-                    const double* rr = s->rhoT.data() + ((size_t)(s->dmd ? b * nt + a : a * nt + b) * nr + m) * 8;
-                    for (int k = 0; k < 4; k++) dst[k] = rr[k];
-                    if (a >= b || !s->dmd) {
-                        const double* pp = s->phiT.data() + ((size_t)comp_idx(a, b) * nr + m) * 8;
-                        for (int k = 0; k < 4; k++) dst[4 + k] = pp[k];
+            for (int b = 0; b < nt; b++) {
+                double* dst = pk64.get() + (size_t)(a * nt + b) * nr * 8;
+                const double* rr = s->rhoT.data() + (size_t)(s->dmd ? b * nt + a : a * nt + b) * nr * 8;
+                const double* pp = s->phiT.data() + (size_t)comp_idx(a, b) * nr * 8;
+                const bool with_phi = a >= b || !s->dmd;
+                for (int m = 0; m < nr; m++, dst += 8, rr += 8, pp += 8)
+                    for (int k = 0; k < 4; k++) {
+                        dst[k] = rr[k];
+                        dst[4 + k] = with_phi ? pp[k] : 0.0;
                     }
-                }
-        CHK(dalloc(&s->d_pk64, pk64.size()));
-        CU(cudaMemcpy(s->d_pk64, pk64.data(), pk64.size() * sizeof(double), cudaMemcpyHostToDevice));
+            }
+        CHK(dalloc(&s->d_pk64, np));
+        CU(cudaMemcpy(s->d_pk64, pk64.get(), np * sizeof(double), cudaMemcpyHostToDevice));
         d.pk64 = s->d_pk64;
     }
     if (s->dmd) {
