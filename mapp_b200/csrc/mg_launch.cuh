@@ -2,8 +2,9 @@
 //
 // The library's calls are chains of short kernels, and at small sizes the gaps
 // between them (the next grid is set up only when the last block of the one
-// before has drained) cost as much as the kernels: 68 us for the 17 kernels of a
-// BDF clock's iteration at 500 sites (56 us with overlapping starts).  A kernel queued by launch_dep is set up
+// before has drained) cost as much as the kernels.  c_d_calc and calc_g, sixteen
+// kernels in all: 182 us with plain launches and 171 with overlapping starts at
+// 2048 sites, 312 and 288 at 32000.  A kernel queued by launch_dep is set up
 // while the one before it runs; its blocks wait in dep_sync, its first
 // statement, until everything before it in the stream is complete and visible.
 // (Two kernels split dep_sync: k_mlp_train reads its rows before the wait and
@@ -58,12 +59,18 @@ inline cudaError_t launch_dep(void (*kern)(P...), unsigned grid, unsigned block,
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// A persistent kernel whose resident blocks fill the SMs' shared memory: queued
-// with an overlapping start only while its grid is at most one block per SM.  A
-// full grid set up beside the blocks of a kernel that left most of the SM to the
-// L1 does not find the shared memory for all its blocks and runs in two rounds
-// (precision form, 256000 sites: 772 us a call instead of 604 us; the learned
-// form's kernels, 108000 sites: 1551 us instead of 1508 us).
+// For the precision and learned forms' persistent kernels: queued with an
+// overlapping start only while the grid is at most one block per SM.  Most of
+// them keep the potential tables or the network in shared memory, as many blocks
+// an SM as that allows, and a full grid set up beside the blocks of a kernel that
+// left most of the SM to the L1 does not find the shared memory for all its blocks
+// and runs in two rounds: precision form, 256000 sites, k_dmd32_dens and
+// k_dmd32_force queued early 780-810 us a call instead of 630.  Kernels that live
+// off the L1 (the EAM, FS and plain DMD passes) are queued by launch_dep with full
+// grids: 256000 atoms 351 us instead of 353-358, 256000 sites 1412 instead of
+// 1423-1431.  The learned form's k_mlp_rows, k_mlp_densities and k_dmd32_pass2 stand
+// between the two; queued early they make no difference (62500 sites 953-980 us, 957-962
+// plainly; 500000 sites 6325-6374 and 6336-6348), so they go with their neighbours.
 template <typename... P>
 inline cudaError_t launch_full(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
                                 typename same_type<P>::type... args)
