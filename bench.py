@@ -1046,7 +1046,9 @@ def run_ours(args):
         # reduction; precision prep, density, embedding, force, merge,
         # reduction; learned rows, fallback, network, audit, densities,
         # embedding, pass 2, reduction
-        "gpu_launches": {"fp64": 4, "fp32": 6, "mlp": 8}[args.form] * args.steps,
+        # per force_calc: the zeroing of the sums (not the precision form, whose first
+        # kernel does it), the form's passes, the reduction of the totals
+        "gpu_launches": {"fp64": 5, "fp32": 6, "mlp": 9}[args.form] * args.steps,
         "phases_ms": {"force": t_dev / args.steps, "force.pass1": p1_ms, "force.embed": emb_ms,
                       "force.pass2": p2_ms, "force_with_phase_events": t_dev_phased,
                       "phase_note": "per-kernel times from a second loop of the same steps with the library's "
