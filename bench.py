@@ -1042,12 +1042,10 @@ def run_ours(args):
                 "client_energy_rel_diff": (abs(e2e_client["energy"] - float(en_py[0])) / abs(float(en_py[0]))
                                            if e2e_client else None)},
         "forms": forms,
-        # library kernels per force call: plain pass 1, embedding, pass 2,
-        # reduction; precision prep, density, embedding, force, merge,
-        # reduction; learned rows, fallback, network, audit, densities,
-        # embedding, pass 2, reduction
-        # per force_calc: the zeroing of the sums (not the precision form, whose first
-        # kernel does it), the form's passes, the reduction of the totals
+        # library kernels per force call: plain zeroing, pass 1, embedding, pass 2,
+        # reduction; precision prep (which zeroes), density, embedding, force,
+        # merge, reduction; learned zeroing, rows, fallback, network, audit,
+        # densities, embedding, pass 2, reduction
         "gpu_launches": {"fp64": 5, "fp32": 6, "mlp": 9}[args.form] * args.steps,
         "phases_ms": {"force": t_dev / args.steps, "force.pass1": p1_ms, "force.embed": emb_ms,
                       "force.pass2": p2_ms, "force_with_phase_events": t_dev_phased,
